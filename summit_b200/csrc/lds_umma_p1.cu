@@ -16,6 +16,8 @@
 // per TMEM lane quadrant) read the accumulator out and split it into digits.  Two TMEM accumulators let the MMAs of the next job (super-bin,
 // column group) run while the epilogue of the previous one drains, which
 // matters for windowed estimates, whose super-bins are a few K-steps long.
+#include <algorithm>
+#include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
 
@@ -382,96 +384,190 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
 
 // Weight digits in the layout of p1_umma_kernel:
 // Wq[((k*2 + part)*ncolp + 4 v + t)*Lmax + r], part 0 = W1, 1 = -W2.
-// One CTA per (k, v); padding entries are left as zero (buffer cleared once).
-__global__ void p1_weights4_kernel(P1UWeights w, const double* __restrict__ mean,
-                                   const double* __restrict__ sdinv, const double* __restrict__ Z,
-                                   int64_t z_ld) {
-    __shared__ double red[32];
-    const int k = blockIdx.x / w.V, v = blockIdx.x - (blockIdx.x / w.V) * w.V;
+// Entries past a list's padded length are never read.
+//
+// Latency-bound gathers (rowind -> sdinv, mean, Z) followed by 8 bytes written
+// per (member, probe).  A cluster of CTAs owns a (bin, probe) column: each CTA
+// a slice of the members, 4 consecutive members per thread (one 4-byte store
+// per digit after a byte transpose), the column's maximum and bound through
+// distributed shared memory.  A thread's first four weights stay in registers
+// between the two passes, which covers lists of up to 4 threads-widths without
+// a second gather.  The value's 28 bits are rounded once and split by
+// digits_word.  K = 1, V = 20, 20,000 members: 95 -> 15 us; V = 50, 16,001
+// members: 112 -> 25 us (one 256-thread CTA per column, byte stores, FP64
+// digit splitting).
+// Short lists (windowed super-bins) take a warp per column instead, 8 columns
+// per CTA, so that an SM has 24 and not 5 of their gather chains in flight
+// (966 super-bins x 50 probes of 128 to 640 members: 326 -> 123 us).
+constexpr int kWMaxThreads = 512;
+constexpr int kWShort = 1024;     // longest list of the warp form
+constexpr int kWWarps = 8;        // its columns per CTA
+
+template <bool kWarp>
+__global__ void __launch_bounds__(kWarp ? 32 * kWWarps : kWMaxThreads)
+    p1_weights4_kernel(P1UWeights w, const double* __restrict__ mean,
+                       const double* __restrict__ sdinv, const double* __restrict__ Z,
+                       int64_t z_ld) {
+    __shared__ double red[2][kWMaxThreads / 32];
+    __shared__ double c_red[2];   // slice maximum and bound, read by the cluster
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (int)(blockDim.x >> 5);
+    const int nranks = kWarp ? 1 : (int)cl.num_blocks(), rank = kWarp ? 0 : (int)cl.block_rank();
+    const int64_t kv = kWarp ? (int64_t)blockIdx.x * kWWarps + warp : (int64_t)(blockIdx.x / nranks);
+    if (kWarp && kv >= (int64_t)w.K * w.V) return;
+    const int gtid = kWarp ? lane : (int)threadIdx.x;       // thread of this column's group
+    const int gsize = kWarp ? 32 : (int)blockDim.x;
+    const int k = (int)(kv / w.V), v = (int)(kv - (int64_t)k * w.V);
     const int64_t r0 = w.bin_off[k], nnzp = w.bin_off[k + 1] - r0;
-    double amax = 0.0;
-    for (int64_t r = threadIdx.x; r < nnzp; r += blockDim.x) {
-        const double sc = w.sc[r0 + r];
-        if (sc == 0.0) continue;
-        const int64_t j = w.rowind[r0 + r];
-        const double w1 = sdinv[j] * (sc * Z[(int64_t)v * z_ld + j]);
-        amax = fmax(amax, fmax(fabs(w1), fabs(mean[j] * w1)));
+    const int64_t stride = (int64_t)nranks * gsize * 4;
+    const int64_t rbeg = ((int64_t)rank * gsize + gtid) * 4;
+    // Members r .. r + 3 (lists are padded to a multiple of 128): w1 and mu w1.
+    auto load4 = [&](int64_t r, double (&a)[4], double (&m)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double sc = w.sc[r0 + r + q];
+            a[q] = m[q] = 0.0;
+            if (sc != 0.0) {
+                const int64_t j = w.rowind[r0 + r + q];
+                a[q] = sdinv[j] * (sc * Z[(int64_t)v * z_ld + j]);
+                m[q] = mean[j] * a[q];
+            }
+        }
+    };
+    double a0[4] = {0, 0, 0, 0}, m0[4] = {0, 0, 0, 0};
+    double amax = 0.0, bsum = 0.0;
+    for (int64_t r = rbeg; r < nnzp; r += stride) {
+        double a[4], m[4];
+        load4(r, a, m);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            amax = fmax(amax, fmax(fabs(a[q]), fabs(m[q])));
+            bsum += 2.0 * fabs(a[q]) + fabs(m[q]);
+            if (r == rbeg) {
+                a0[q] = a[q];
+                m0[q] = m[q];
+            }
+        }
     }
-    for (int o = 16; o; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double x = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0;
-        for (int o = 16; o; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-        if (threadIdx.x == 0) red[0] = x;
+    for (int o = 16; o; o >>= 1) {
+        amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
     }
-    __syncthreads();
-    amax = red[0];
+    if (!kWarp) {
+        if (lane == 0) {
+            red[0][warp] = amax;
+            red[1][warp] = bsum;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            double x = lane < nwarps ? red[0][lane] : 0.0, y = lane < nwarps ? red[1][lane] : 0.0;
+            for (int o = 16; o; o >>= 1) {
+                x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+                y += __shfl_xor_sync(0xffffffffu, y, o);
+            }
+            if (lane == 0) {
+                c_red[0] = x;
+                c_red[1] = y;
+            }
+        }
+        if (nranks == 1) {
+            __syncthreads();
+            amax = c_red[0];
+            bsum = c_red[1];
+        } else {
+            cl.sync();
+            amax = bsum = 0.0;
+            for (int q = 0; q < nranks; ++q) {
+                amax = fmax(amax, *cl.map_shared_rank(&c_red[0], q));
+                bsum += *cl.map_shared_rank(&c_red[1], q);
+            }
+        }
+    }
     int e = 0;
     if (amax > 0.0 && isfinite(amax)) {
         e = ilogb(amax) + 1;
         if (ldexp(amax, 7 - e) > 127.0) e += 1;
     }
+    // 2^(28 - e) as two factors: it overflows for columns of tiny weights.
+    const int e1 = min(28 - e, 1000);
+    const double f1 = ldexp(1.0, e1), f2 = ldexp(1.0, 28 - e - e1);
     int8_t* b1 = w.wq + ((int64_t)(k * 2 + 0) * w.ncolp + 4 * v) * w.lmax;
     int8_t* b2 = w.wq + ((int64_t)(k * 2 + 1) * w.ncolp + 4 * v) * w.lmax;
-    for (int64_t r = threadIdx.x; r < nnzp; r += blockDim.x) {
-        const double sc = w.sc[r0 + r];
-        double t1 = 0.0, t2 = 0.0;
-        if (sc != 0.0) {
-            const int64_t j = w.rowind[r0 + r];
-            const double w1 = sdinv[j] * (sc * Z[(int64_t)v * z_ld + j]);
-            t1 = ldexp(w1, 7 - e);
-            t2 = ldexp(-(mean[j] * w1), 7 - e);
-        }
+    for (int64_t r = rbeg; r < nnzp; r += stride) {
+        double a[4], m[4];
+        if (r == rbeg) {
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const double q1 = rint(t1), q2 = rint(t2);
-            b1[(int64_t)s * w.lmax + r] = (int8_t)q1;
-            b2[(int64_t)s * w.lmax + r] = (int8_t)q2;
-            t1 = (t1 - q1) * 128.0;
-            t2 = (t2 - q2) * 128.0;
+            for (int q = 0; q < 4; ++q) {
+                a[q] = a0[q];
+                m[q] = m0[q];
+            }
+        } else {
+            load4(r, a, m);
         }
+        uint32_t x[4], d[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = digits_word(__double2int_rn(a[q] * f1 * f2));
+        transpose4x4(x[0], x[1], x[2], x[3], d[3], d[2], d[1], d[0]);  // byte b: digit 3 - b
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            *reinterpret_cast<uint32_t*>(b1 + (int64_t)s * w.lmax + r) = d[s];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = digits_word(__double2int_rn(-(m[q] * f1 * f2)));
+        transpose4x4(x[0], x[1], x[2], x[3], d[3], d[2], d[1], d[0]);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            *reinterpret_cast<uint32_t*>(b2 + (int64_t)s * w.lmax + r) = d[s];
     }
-    if (threadIdx.x == 0) w.colscale[(int64_t)k * w.V + v] = ldexp(1.0, e - 7 - 21);
-    if (w.ycolscale) {
-        // Rigorous bound on |y_i| = |sum_j g_ij w1_j - o_ij w2_j| <= sum_j 2|w1_j| + |w2_j|
-        // (inflated for the digit rounding of the weights), fixing the sketch's
-        // digit exponent before phase 1 runs.
-        double bsum = 0.0;
-        for (int64_t r = threadIdx.x; r < nnzp; r += blockDim.x) {
-            const double sc = w.sc[r0 + r];
-            if (sc == 0.0) continue;
-            const int64_t j = w.rowind[r0 + r];
-            const double w1 = sdinv[j] * (sc * Z[(int64_t)v * z_ld + j]);
-            bsum += 2.0 * fabs(w1) + fabs(mean[j] * w1);
-        }
-        __syncthreads();
-        for (int o = 16; o; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = bsum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double tot = 0.0;
-            for (int q = 0; q < (int)(blockDim.x >> 5); ++q) tot += red[q];
-            // The weights enter as 4-digit values, each within 2^(e-29) of w1 and
-            // of mu*w1: add that slack for every member, then the FP64 rounding
-            // of the sum.
-            tot = (tot + (double)nnzp * 3.0 * ldexp(1.0, e - 29)) * (1.0 + 1e-9);
+    if (rank == 0 && gtid == 0) {
+        w.colscale[kv] = ldexp(1.0, e - 7 - 21);
+        if (w.ycolscale) {
+            // Rigorous bound on |y_i| = |sum_j g_ij w1_j - o_ij w2_j| <= sum_j 2|w1_j| + |w2_j|,
+            // fixing the sketch's digit exponent before phase 1 runs.  The weights enter as
+            // 4-digit values, each within 2^(e-29) of w1 and of mu*w1: add that slack for
+            // every member, then the FP64 rounding of the sum.
+            const double tot = (bsum + (double)nnzp * 3.0 * ldexp(1.0, e - 29)) * (1.0 + 1e-9);
             int ey = 0;
             if (tot > 0.0 && isfinite(tot)) {
                 ey = ilogb(tot) + 1;
                 if (ldexp(tot, 7 - ey) > 127.0) ey += 1;
             }
-            w.ycolscale[(int64_t)k * w.V + v] = ldexp(1.0, ey - 28);
+            w.ycolscale[kv] = ldexp(1.0, ey - 28);
             // digit shift for the phase-1 epilogue: R = rint(T 2^(eW - eY))
-            w.yshift[(int64_t)k * w.V + v] = e - ey;
+            w.yshift[kv] = e - ey;
         }
     }
+    if (nranks > 1) cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
 void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* sdinv,
                         const double* Z, int64_t z_ld, cudaStream_t st) {
-    if (w.K * w.V == 0) return;
-    p1_weights4_kernel<<<(unsigned)(w.K * w.V), 256, 0, st>>>(w, mean, sdinv, Z, z_ld);
+    const int64_t kv = (int64_t)w.K * w.V;
+    if (kv == 0) return;
+    if (w.lmax <= kWShort && kv >= 148 * kWWarps) {
+        p1_weights4_kernel<true><<<(unsigned)((kv + kWWarps - 1) / kWWarps), 32 * kWWarps, 0, st>>>(
+            w, mean, sdinv, Z, z_ld);
+        count_launch();
+        return;
+    }
+    // As many threads as the longest list has groups of 4 members, and a
+    // cluster where that is more than a CTA's and the columns alone leave SMs
+    // without a CTA.
+    const int64_t quads = (w.lmax + 3) / 4;
+    const int threads = (int)std::min<int64_t>(kWMaxThreads, (quads + 31) / 32 * 32);
+    int width = 1;
+    while (width < 8 && kv * width < 2 * 148 && quads > (int64_t)threads * width) width *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(kv * width));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)width;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, p1_weights4_kernel<false>, w, mean, sdinv, Z, z_ld);
     count_launch();
 }
 
