@@ -119,6 +119,7 @@ struct P1UArgs {
     double* Y = nullptr;                // N_pad x (K*V), column (k*V+v)
     unsigned int* status = nullptr;
     int sb_per_cta = 1;                 // super-bins processed by one CTA (pipeline continues)
+    int nsplit = 1;                     // CTAs that share a super-bin's K-steps (FP64 output only)
     // Digit output (windowed estimates): when yq is set the epilogue writes the
     // sketch's 4 int8 digits in phase 2's layout (digit_offset, column
     // k*ncolp + 4v + t of K*ncolp) using the a-priori exponents in ycolscale
@@ -143,7 +144,7 @@ struct P1UWeights {
 
 void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* sdinv,
                         const double* Z, int64_t z_ld, cudaStream_t st);
-size_t p1_umma_smem_bytes();
+size_t p1_umma_smem_bytes(int box_rows);
 void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cudaStream_t st);
 
 // Columns per bin (4 digits per probe, padded to a multiple of 16).

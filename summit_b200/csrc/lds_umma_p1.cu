@@ -9,13 +9,19 @@
 // TMA, SWIZZLE_128B, K-major) into ONE accumulator, so TMEM holds
 // G.W1 - O.W2 = sum_j (g - mu_j o) s_j sc z directly.
 //
-// Roles (704 threads): warp 0 TMA producer for the digit tiles; warp 1 TMEM
-// allocation and the single MMA-issuing thread; warps 2-5 gather the member
-// SNPs' packed bytes from global memory (one row each, kept several stages
-// ahead by cp.async) and decode them into the operand tiles; warps 6-21 (four
-// per TMEM lane quadrant) read the accumulator out and split it into digits.  Two TMEM accumulators let the MMAs of the next job (super-bin,
-// column group) run while the epilogue of the previous one drains, which
-// matters for windowed estimates, whose super-bins are a few K-steps long.
+// Roles (832 threads): warp 0 TMA producer for the digit tiles; warp 1 TMEM
+// allocation and the single MMA-issuing thread; warps 2-9, two decoder sets of
+// four (set d takes the K-steps of its parity), gather the member SNPs' packed
+// bytes from global memory (one row each, kept several steps ahead by
+// cp.async) and decode them into the operand tiles; warps 10-25 (four per TMEM
+// lane quadrant) read the accumulator out and split it into digits.  Two TMEM
+// accumulators let the MMAs of the next job (super-bin, column group) run while
+// the epilogue of the previous one drains, which matters for windowed
+// estimates, whose super-bins are a few K-steps long.
+//
+// What bounds it: with many K-steps per super-bin the decode (one set of four
+// warps held a K-step at 2,007 cycles against 832 of MMA at N = 208); with few,
+// the digit epilogue's instructions per (sample, probe).
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -29,52 +35,90 @@ namespace lds {
 namespace umma {
 
 namespace p1 {
-constexpr int kStages = 2;
+constexpr int kMaxStages = 4;
 constexpr int kBM = 128;          // samples per CTA
 constexpr int kBK = 128;          // member SNPs per stage
 constexpr int kATile = 128 * 128; // 16 KB
-constexpr int kWTile = 256 * 128; // 32 KB (max digit columns per pass)
-constexpr int kStageBytes = 2 * kATile + 2 * kWTile;  // 96 KB
-constexpr int kThreads = 704;
-constexpr int kEpiThreads = 512;         // warps 6..21: four per TMEM lane quadrant
+constexpr int kDecSets = 2;
+constexpr int kDecWarp0 = 2;
+constexpr int kEpiWarp0 = kDecWarp0 + 4 * kDecSets;
+constexpr int kEpiWarps = 16;            // four per TMEM lane quadrant
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 constexpr int kAccCols = 256;            // one accumulator: <= 256 digit columns
 constexpr uint32_t kTmemCols = 512;      // two accumulators (MMA of job j+1 || epilogue of j)
-constexpr int kRing = 6;                 // gathered packed rows in flight per decoder thread
+constexpr int kRing = 6;                 // K-steps whose packed rows are in flight
 constexpr int kRingSlot = 128 * 32;      // 128 member rows x 32 bytes
+constexpr int kMaxSb = 256;              // super-bins per CTA (their offsets in shared memory)
+constexpr int kSmemLimit = 227 * 1024;
+// Longest list whose |128 t2 + t3| stays below 2^31: the low digits' products
+// are at most 3 * 64 per member.
+constexpr int kMaxNarrowSteps = 86000 / kBK;
+
+// Shared memory: the stages (G and O tiles, then the two weight-digit tiles of
+// box_rows columns), the gather ring, the barriers, the super-bin table, and
+// each epilogue warp's digit-shift table.
+struct Layout {
+    uint32_t w_tile, stage;
+    int stages;
+    __host__ __device__ explicit Layout(int box_rows)
+        : w_tile((uint32_t)((box_rows * kBK + 1023) / 1024 * 1024)),
+          stage(2 * kATile + 2 * w_tile),
+          stages(0) {
+        const int fit = (int)((kSmemLimit - 1024 - tail()) / stage);
+        stages = fit < kMaxStages ? fit : kMaxStages;
+    }
+    __host__ __device__ static constexpr uint32_t tail() {
+        return kRing * kRingSlot + 256 + (kMaxSb + 4) * 4 + kEpiWarps * 16 * 16;
+    }
+    __host__ __device__ uint32_t ring_off() const { return (uint32_t)stages * stage; }
+    __host__ __device__ uint32_t bar_off() const { return ring_off() + kRing * kRingSlot; }
+    __host__ __device__ uint32_t shift_off() const { return bar_off() + 256; }
+    __host__ __device__ uint32_t table_off() const { return shift_off() + kEpiWarps * 16 * 16; }
+    __host__ __device__ uint32_t bytes() const { return ring_off() + tail(); }
+};
+static_assert(2 * (2 * kATile + 2 * 256 * kBK) + Layout::tail() + 1024 <= kSmemLimit,
+              "two stages of 256 digit columns fit");
 }  // namespace p1
 
 __global__ void __launch_bounds__(p1::kThreads, 1)
     p1_umma_kernel(const __grid_constant__ CUtensorMap tmW, P1UArgs a) {
     using namespace p1;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* ring = smem + kStages * kStageBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kRing * kRingSlot);
-    uint64_t* full_w = bars;                    // [kStages] weight tiles landed (TMA)
-    uint64_t* full_dec = bars + kStages;        // [kStages] genotype tiles decoded
-    uint64_t* empty = bars + 2 * kStages;       // [kStages] stage consumed by the MMAs
-    uint64_t* acc_full = bars + 3 * kStages;    // [2] accumulator b holds a finished job
+    uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
+    const Layout lay(a.box_rows);
+    const int nst = lay.stages;
+    uint8_t* ring = smem + lay.ring_off();
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off());
+    uint64_t* full_w = bars;                    // [nst] weight tiles landed (TMA)
+    uint64_t* full_dec = bars + kMaxStages;     // [nst] genotype tiles decoded
+    uint64_t* empty = bars + 2 * kMaxStages;    // [nst] stage consumed by the MMAs
+    uint64_t* acc_full = bars + 3 * kMaxStages; // [2] accumulator b holds a finished job
     uint64_t* acc_empty = acc_full + 2;         // [2] accumulator b read out
     uint64_t* mma_done = acc_empty + 2;         // drain of the issuer's MMAs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int4* shift_tab = reinterpret_cast<int4*>(smem + lay.shift_off());
+    int* ktab = reinterpret_cast<int*>(smem + lay.table_off());
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t i0 = (int64_t)blockIdx.x * kBM;
-    // This CTA's super-bins: [kb0, kb1); a job is one (super-bin, column group).
+    // This CTA's super-bins: kb0 .. kb0 + nsb; a job is one (super-bin, column
+    // group).  ktab holds their list offsets in K-steps.  With nsplit > 1 the CTA
+    // takes part blockIdx.z of every super-bin's K-steps.
     const int kb0 = blockIdx.y * a.sb_per_cta;
-    const int kb1 = min(a.K, kb0 + a.sb_per_cta);
+    const int nsb = min(a.K - kb0, a.sb_per_cta);
 
+    for (int q = tid; q <= nsb; q += kThreads) ktab[q] = (int)(a.bin_off[kb0 + q] / kBK);
     if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < nst; ++s) {
             mbar_init(&full_w[s], 1);
-            mbar_init(&full_dec[s], 4);            // one arrival per decoder warp
+            mbar_init(&full_dec[s], 4);            // one arrival per decoder warp of the step's set
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], kEpiThreads / 32);  // one arrival per epilogue warp
+            mbar_init(&acc_empty[b], kEpiWarps);   // one arrival per epilogue warp
         }
         mbar_init(mma_done, 1);
         *abort_flag = 0;
@@ -94,40 +138,52 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         atomicCAS(a.status, 0u, (unsigned)code);
         *abort_flag = 1;
     };
-    auto nkt_of = [&](int k) { return (int)((a.bin_off[k + 1] - a.bin_off[k]) / kBK); };
+    // K-steps [k0, k0 + n) of super-bin kb0 + q that this CTA takes.
+    auto steps_of = [&](int q, int& k0) {
+        const int n = ktab[q + 1] - ktab[q];
+        if (a.nsplit <= 1) {
+            k0 = 0;
+            return n;
+        }
+        const int per = (n + a.nsplit - 1) / a.nsplit;
+        k0 = min(n, (int)blockIdx.z * per);
+        return min(n, k0 + per) - k0;
+    };
 
     if (warp == 0) {
         // ---------------- TMA producer of weight-digit tiles ----------------
         if (lane == 0) {
-            int it = 0;
-            for (int k = kb0; k < kb1 && !*abort_flag; ++k) {
-                const int nkt = nkt_of(k);
+            int it = 0, s = 0;
+            uint32_t ph = 0;
+            for (int q = 0; q < nsb && !*abort_flag; ++q) {
+                int k0;
+                const int nkt = steps_of(q, k0);
                 for (int g = 0; g < a.ngroups && !*abort_flag; ++g) {
                     for (int kt = 0; kt < nkt; ++kt, ++it) {
-                        const int s = it % kStages;
-                        const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-                        if (it >= kStages && !mbar_wait(&empty[s], ph ^ 1u)) { fail(11); break; }
+                        if (it >= nst && !mbar_wait(&empty[s], ph ^ 1u)) { fail(11); break; }
                         if (*abort_flag) break;
-                        uint8_t* st = smem + s * kStageBytes;
+                        uint8_t* w = smem + s * lay.stage + 2 * kATile;
                         mbar_expect_tx(&full_w[s], (uint32_t)(2 * a.box_rows * kBK));
-                        const int y0 = k * 2 * a.ncolp + g * 256;
-                        tma_load_2d(st + 2 * kATile, &tmW, kt * kBK, y0, &full_w[s]);
-                        tma_load_2d(st + 2 * kATile + kWTile, &tmW, kt * kBK, y0 + a.ncolp,
-                                    &full_w[s]);
+                        const int y0 = (kb0 + q) * 2 * a.ncolp + g * 256;
+                        tma_load_2d(w, &tmW, (k0 + kt) * kBK, y0, &full_w[s]);
+                        tma_load_2d(w + lay.w_tile, &tmW, (k0 + kt) * kBK, y0 + a.ncolp, &full_w[s]);
+                        if (++s == nst) { s = 0; ph ^= 1u; }
                     }
                 }
             }
             // Drain: no tile copy may still be landing when the CTA exits
             // (only reachable with copies outstanding after an abort).
-            for (int j = max(0, it - kStages); j < it; ++j)
-                mbar_wait(&full_w[j % kStages], (uint32_t)(j / kStages) & 1u);
+            for (int j = max(0, it - nst); j < it; ++j)
+                mbar_wait(&full_w[j % nst], (uint32_t)(j / nst) & 1u);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            int it = 0, au = 0;  // stage counter, jobs (accumulator uses)
-            for (int k = kb0; k < kb1 && !*abort_flag; ++k) {
-                const int nkt = nkt_of(k);
+            int s = 0, au = 0;  // stage, jobs (accumulator uses)
+            uint32_t ph = 0;
+            for (int q = 0; q < nsb && !*abort_flag; ++q) {
+                int k0;
+                const int nkt = steps_of(q, k0);
                 if (nkt == 0) continue;
                 for (int g = 0; g < a.ngroups && !*abort_flag; ++g, ++au) {
                     const int b = au & 1, u = au >> 1;
@@ -136,20 +192,18 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     const uint32_t acc = tmem + (uint32_t)(b * kAccCols);
                     if (u > 0 && !mbar_wait(&acc_empty[b], (uint32_t)(u - 1) & 1u)) { fail(12); break; }
                     tc_fence_after();
-                    for (int kt = 0; kt < nkt; ++kt, ++it) {
-                        const int s = it % kStages;
-                        const uint32_t ph = (uint32_t)(it / kStages) & 1u;
+                    for (int kt = 0; kt < nkt; ++kt) {
                         if (!mbar_wait(&full_dec[s], ph) || !mbar_wait(&full_w[s], ph)) {
                             fail(13);
                             break;
                         }
                         if (*abort_flag) break;
                         tc_fence_after();
-                        uint8_t* st = smem + s * kStageBytes;
+                        uint8_t* st = smem + s * lay.stage;
                         const uint64_t dG = sw128_desc_mn(st);
                         const uint64_t dO = sw128_desc_mn(st + kATile);
                         const uint64_t dW1 = sw128_desc(st + 2 * kATile);
-                        const uint64_t dW2 = sw128_desc(st + 2 * kATile + kWTile);
+                        const uint64_t dW2 = sw128_desc(st + 2 * kATile + lay.w_tile);
 #pragma unroll
                         for (int kk = 0; kk < kBK / 32; ++kk) {
                             // A advances 32 K-rows = 4 swizzle atoms (4 KB); B advances 32 bytes.
@@ -157,6 +211,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                             umma_i8(acc, dO + 256 * kk, dW2 + 2 * kk, idesc, 1u);
                         }
                         umma_commit(&empty[s]);
+                        if (++s == nst) { s = 0; ph ^= 1u; }
                     }
                     umma_commit(&acc_full[b]);
                 }
@@ -165,78 +220,111 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             umma_commit(mma_done);
             mbar_wait(mma_done, 0u);
         }
-    } else if (warp < 6) {
-        // ---------------- gather + decode (warps 2..5) ----------------
-        const int t = tid - 64;
+    } else if (warp < kEpiWarp0) {
+        // ---------------- gather + decode (two sets of four warps) ----------------
+        // Set d decodes the K-steps it with it % 2 == d, so two operand tiles
+        // are in the making while the MMAs read a third.
+        const int dset = (warp - kDecWarp0) >> 2;
+        const int t = (tid - 32 * kDecWarp0) & 127;
         const uint8_t* codes = a.codes + i0 / 4;
         // Gather prefetcher: walks the same (super-bin, group, K-step) sequence
-        // kRing steps ahead, copying this thread's member row into a ring slot.
-        // The member row of the step being fetched is read from rowind one step
-        // earlier (row_next), so that load's latency overlaps a step of work
-        // instead of stalling the cp.async that needs the address.
-        int pk = kb0, pg = 0, pkt = 0, pit = 0;
-        auto cursor_row = [&]() -> int64_t {  // rowind of the cursor's step, or -1 past the end
-            while (pk < kb1 && nkt_of(pk) == 0) { ++pk; pg = 0; pkt = 0; }
-            if (pk >= kb1) return -1;
-            int64_t row = a.rowind[a.bin_off[pk] + (int64_t)pkt * kBK + t];
+        // ahead of the decode, copying this thread's member row of the set's
+        // steps into ring slots.  The member row of the step being fetched is
+        // read from rowind one step earlier (row_next), so that load's latency
+        // overlaps a step of work instead of stalling the cp.async that needs
+        // the address.
+        int pq = -1, pg = a.ngroups - 1, pkt = 0, pn = 0, pit = 0;
+        const int32_t* prow = nullptr;
+        bool pend = false;
+        auto advance = [&]() {   // cursor to the next K-step, or pend past the last one
+            if (pend || pkt < pn) {
+                return;
+            }
+            pkt = 0;
+            if (pn > 0 && ++pg < a.ngroups) return;
+            pg = 0;
+            int k0 = 0;
+            do {
+                if (++pq >= nsb) {
+                    pend = true;
+                    return;
+                }
+                pn = steps_of(pq, k0);
+            } while (pn == 0);
+            prow = a.rowind + ((int64_t)(ktab[pq] + k0) * kBK + t);
+        };
+        auto cursor_row = [&]() -> int64_t {  // member row of the set's next step, or -1
+            advance();
+            if (pend) return -1;
+            if ((pit & 1) != dset) {          // the other set's step
+                ++pkt;
+                ++pit;
+                advance();
+                if (pend) return -1;
+            }
+            int64_t row = prow[(int64_t)pkt * kBK];
             // bounds-checked build: a member row outside the image is not gathered
             if (!in_range(a.m_pad == 0 || (row >= 0 && row < a.m_pad), 0x1001u)) row = -2;
-            if (++pkt == nkt_of(pk)) {
-                pkt = 0;
-                if (++pg == a.ngroups) { pg = 0; ++pk; }
-            }
+            ++pkt;
+            ++pit;
             return row;
         };
+        int pslot = dset;                     // ring slot of the step being fetched
         int64_t row_next = cursor_row();
         auto prefetch_one = [&]() {
             const int64_t row = row_next;
             row_next = cursor_row();
             if (row >= 0) {
                 const uint8_t* src = codes + row * a.nbp;
-                uint8_t* dst = ring + (pit % kRing) * kRingSlot + t * 32;
+                uint8_t* dst = ring + pslot * kRingSlot + t * 32;
                 cp_async16(dst, src);
                 cp_async16(dst + 16, src + 16);
             }
             cp_async_commit();
-            ++pit;
+            pslot = pslot + 2 < kRing ? pslot + 2 : dset;
         };
-        for (int d = 0; d < kRing - 1; ++d) prefetch_one();
-        int it = 0;
-        for (int k = kb0; k < kb1 && !__any_sync(0xffffffffu, *abort_flag != 0); ++k) {
-            const int nkt = nkt_of(k);
-            for (int g = 0; g < a.ngroups && nkt > 0 && !__any_sync(0xffffffffu, *abort_flag != 0); ++g) {
-                for (int kt = 0; kt < nkt; ++kt, ++it) {
-                    const int s = it % kStages;
-                    const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-                    prefetch_one();  // step it + kRing - 1
-                    asm volatile("cp.async.wait_group %0;\n" ::"n"(kRing - 1));
+        constexpr int kDepth = kRing / 2;     // steps of this set in flight
+        for (int d = 0; d < kDepth - 1; ++d) prefetch_one();
+        int it = 0, s = 0, slot = 0;
+        uint32_t ph = 0;
+        for (int q = 0; q < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); ++q) {
+            int k0;
+            const int nkt = steps_of(q, k0) * a.ngroups;
+            for (int kt = 0; kt < nkt; ++kt, ++it) {
+                if ((it & 1) == dset) {
+                    prefetch_one();
+                    asm volatile("cp.async.wait_group %0;\n" ::"n"(kDepth - 1));
                     const uint4* src =
-                        reinterpret_cast<const uint4*>(ring + (it % kRing) * kRingSlot + t * 32);
+                        reinterpret_cast<const uint4*>(ring + slot * kRingSlot + t * 32);
                     const uint4 c0 = src[0], c1 = src[1];
-                    if (it >= kStages && !__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u))) {
+                    if (it >= nst && !__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u))) {
                         fail(14);
                         break;
                     }
                     if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
-                    uint8_t* st = smem + s * kStageBytes;
-                    uint8_t* gRow = st + (t >> 3) * 1024 + (t & 7) * 128;
+                    uint8_t* gRow = smem + s * lay.stage + (t >> 3) * 1024 + (t & 7) * 128;
                     decode_row_sw128(c0, c1, gRow, gRow + kATile, t);
                     fence_async_smem();
                     __syncwarp();  // orders the warp's operand stores before its one arrival
                     if (lane == 0) mbar_arrive(&full_dec[s]);
                 }
+                if (++s == nst) { s = 0; ph ^= 1u; }
+                if (++slot == kRing) slot = 0;
             }
         }
         cp_async_wait_all();  // no gather copy may outlive the CTA (abort path)
     } else {
-        // ---------------- epilogue (warps 6..21) ----------------
-        const int e = tid - 192;
+        // ---------------- epilogue (four warps per TMEM lane quadrant) ----------------
+        const int e = tid - 32 * kEpiWarp0;
         const int q = warp & 3;                  // TMEM lane quadrant of this warp
-        const int h = (warp - 6) >> 2;           // which quarter of the 16-column chunks
+        const int h = (warp - kEpiWarp0) >> 2;   // which quarter of the column chunks
         const int64_t i = i0 + q * 32 + lane;    // sample row of this thread's accumulator lane
+        int4* const tab = shift_tab + (warp - kEpiWarp0) * 16;   // this warp's digit shifts
         int au = 0;
-        for (int k = kb0; k < kb1 && !__any_sync(0xffffffffu, *abort_flag != 0); ++k) {
-            const int nkt = nkt_of(k);
+        for (int kq = 0; kq < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); ++kq) {
+            const int k = kb0 + kq;
+            int k0;
+            const int nkt = steps_of(kq, k0);
             // This sample tile's block of super-bin k in phase 2's digit layout
             // (digit_offset): ncolp rows of 128 bytes.
             int8_t* const yblk =
@@ -250,35 +338,43 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             }
             if (nkt == 0) {
                 // Bin without members: its sketch columns are zero (the
-                // reference's untouched-bin zeroing, gw_ldscore.py:2017-2019).
+                // reference's untouched-bin zeroing, gw_ldscore.py:2017-2019;
+                // a split's columns start at zero).
                 if (a.yq) {
                     for (int idx = e; idx < 4 * a.V * 8; idx += kEpiThreads)
                         *reinterpret_cast<uint4*>(yblk + (idx >> 3) * 128 + (idx & 7) * 16) =
                             make_uint4(0, 0, 0, 0);
-                } else {
+                } else if (a.nsplit <= 1) {
                     for (int idx = e; idx < a.V * 64; idx += kEpiThreads)
                         *reinterpret_cast<uint4*>(a.Y + ((int64_t)k * a.V + (idx >> 6)) * a.N_pad +
                                                   i0 + (idx & 63) * 2) = make_uint4(0, 0, 0, 0);
                 }
                 continue;
             }
+            // (nkt is this super-bin's whole list: the digit form is never split)
+            const bool small_sums = nkt <= kMaxNarrowSteps;
             for (int g = 0; g < a.ngroups && !__any_sync(0xffffffffu, *abort_flag != 0); ++g, ++au) {
                 const int b = au & 1, u = au >> 1;
-                // This group's 64 per-probe shifts (or scales), two per lane, loaded
-                // before the accumulator wait so the loads overlap the MMAs; the
-                // loop below broadcasts them with shuffles (warp-local, no barrier).
-                int shA = 0, shB = 0;
+                // Loaded before the accumulator wait so the loads overlap the MMAs:
+                // the digit shifts of this warp's (at most two) chunks of 8 probes,
+                // or the group's 64 per-probe scales, two per lane.
+                bool narrow = false;
                 double scA = 0.0, scB = 0.0;
-                {
+                if (a.yq) {
+                    const int vl = 8 * (h + 4 * ((lane >> 3) & 1)) + (lane & 7);
+                    const int v = g * 64 + vl;
+                    const int r = v < a.V ? -a.yshift[(int64_t)k * a.V + v] : 0;
+                    narrow = small_sums && __all_sync(0xffffffffu, r >= 0 && r <= 14);
+                    // x = right shift, y = 14 - x, z = half an ulp less one, w = parity mask
+                    if (lane < 16)
+                        tab[lane] = make_int4(r, 14 - r, r > 0 ? (1 << ((r - 1) & 15)) - 1 : 0,
+                                              r > 0 ? 1 : 0);
+                    __syncwarp();
+                } else {
                     const int va = g * 64 + lane, vb = va + 32;
                     const int64_t o = (int64_t)k * a.V;
-                    if (a.yq) {
-                        if (va < a.V) shA = a.yshift[o + va];
-                        if (vb < a.V) shB = a.yshift[o + vb];
-                    } else {
-                        if (va < a.V) scA = a.colscale[o + va];
-                        if (vb < a.V) scB = a.colscale[o + vb];
-                    }
+                    if (va < a.V) scA = a.colscale[o + va];
+                    if (vb < a.V) scB = a.colscale[o + vb];
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (uint32_t)u & 1u))) {
                     fail(15);
@@ -292,60 +388,63 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     // digit columns) per TMEM load; the quadrant's four warps take
                     // every fourth chunk.  With y = T 2^(eW-28) and the column
                     // exponent eY fixed in advance by a bound on |y|, the sketch's
-                    // 28-bit value is R = rint(T 2^(eW-eY)) (round half to even);
-                    // its balanced base-128 digits are exact integer work.  A 4 x 4
-                    // byte transpose within each lane quad turns the lanes' digit
-                    // words (4 digits of one sample) into words of one digit for 4
-                    // consecutive samples, stored straight to global memory (a warp
-                    // writes 4 digit rows x 32 samples per probe).  Lane 4a + t
-                    // stores digit row 4v + t, samples s = 32 q + 4a of the block:
-                    // 16-byte chunk s / 16 = 2q + a / 4, swizzled with the row's
-                    // low three bits, (4 v + t) & 7 = 4 (v & 1) + t.
+                    // 28-bit value is R = rint(T 2^-r), r = eY - eW (round half to
+                    // even), and digits_word splits it.  A 4 x 4 byte transpose
+                    // within each lane quad turns the lanes' digit words (4 digits
+                    // of one sample) into words of one digit for 4 consecutive
+                    // samples, stored straight to global memory (a warp writes 4
+                    // digit rows x 32 samples per probe).  Lane 4a + t stores digit
+                    // row 4v + t, samples s = 32 q + 4a of the block: 16-byte chunk
+                    // s / 16 = 2q + a / 4, swizzled with the row's low three bits,
+                    // (4 v + t) & 7 = 4 (v & 1) + t.
+                    //
+                    // R in 32 bits (`narrow`): T = H 2^14 + L with H = 128 t0 + t1 and
+                    // L = 128 t2 + t3 (|L| < 2^31 up to kMaxNarrowSteps K-steps), so for
+                    // 0 <= r <= 14 R = H 2^(14-r) + rint(L 2^-r), the tie parity taken
+                    // from the whole value; H's multiple may wrap, R does not.  19
+                    // instructions per (sample, probe) instead of the 64-bit form's ~60.
                     const int qd = lane & 3;
-                    const uint32_t selA = qd < 2 ? 0x5410u : 0x3276u;
-                    const uint32_t selB = (qd & 1) ? 0x3715u : 0x6240u;
+                    // word byte b holds digit 3 - b: lane t of a quad keeps byte 3 - t
+                    const uint32_t selA = qd < 2 ? 0x7632u : 0x1054u;
+                    const uint32_t selB = (qd & 1) ? 0x2604u : 0x7351u;
                     const int chunk = 2 * q + (lane >> 4);
                     int8_t* const ylane = yblk + qd * 128 + 4 * ((lane >> 2) & 3);
-                    for (int c0 = 32 * h; c0 < ncols; c0 += 128) {
+                    int8_t* const ydst[2] = {ylane + ((chunk ^ qd) << 4),
+                                             ylane + ((chunk ^ (4 + qd)) << 4)};
+                    for (int c0 = 32 * h, cc = 0; c0 < ncols; c0 += 128, cc += 8) {
                         int rr[32];
                         tmem_ld32(tbase + (uint32_t)c0, rr);
                         tmem_wait_ld();
-                        const int vl0 = c0 >> 2;                    // first probe of the chunk
-                        const int nv = a.V - (g * 64 + vl0);        // probes left (warp-uniform)
-#pragma unroll
-                        for (int p = 0; p < 8; ++p) {
-                            const int vl = vl0 + p;
-                            const int sh = __shfl_sync(0xffffffffu, vl < 32 ? shA : shB, vl & 31);
-                            const long long T =
-                                (((long long)rr[4 * p] * 128 + rr[4 * p + 1]) * 128 +
-                                 rr[4 * p + 2]) * 128 + rr[4 * p + 3];
-                            long long R;
-                            if (sh >= 0) {
-                                R = T << sh;
-                            } else {
-                                const int r = -sh;
-                                R = (T + ((1LL << (r - 1)) - 1) + ((T >> r) & 1)) >> r;
-                            }
-                            // |R| < 2^28 (the bound fixed eY): with U = R + 63 (2^14 +
-                            // 2^7 + 1) the low three base-128 digits of U are the
-                            // balanced digits d1..d3 (in [-63, 64]) plus 63 and U >> 21
-                            // is d0; the byte-wise subtraction of 63 from bytes 1..3
-                            // (their top bits set first, so no byte borrows) leaves
-                            // the word [d0, d1, d2, d3].
-                            const int U = (int)R + 63 * (16384 + 128 + 1);
-                            uint32_t w = (uint32_t)(U >> 21) & 0xFFu;
-                            w |= ((uint32_t)(U >> 14) & 127u) << 8;
-                            w |= ((uint32_t)(U >> 7) & 127u) << 16;
-                            w |= ((uint32_t)U & 127u) << 24;
-                            w = ((w | 0x80808000u) - 0x3F3F3F00u) ^ 0x80808000u;
-                            // 4 x 4 byte transpose across the quad: lane 4a + t ends
-                            // with digit t of samples 4a .. 4a + 3.
+                        const int v0 = g * 64 + (c0 >> 2);          // first probe of the chunk (even)
+                        const int nv = a.V - v0;                    // probes left (warp-uniform)
+                        auto store = [&](int p, int R) {
+                            uint32_t w = digits_word(R);
                             w = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 2), selA);
                             w = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 1), selB);
-                            if (p < nv) {
-                                const int v = g * 64 + vl;
-                                *reinterpret_cast<uint32_t*>(
-                                    ylane + v * 512 + ((chunk ^ (4 * (v & 1) + qd)) << 4)) = w;
+                            if (p < nv)
+                                *reinterpret_cast<uint32_t*>(ydst[p & 1] + (int64_t)(v0 + p) * 512) = w;
+                        };
+                        if (narrow) {
+#pragma unroll
+                            for (int p = 0; p < 8; ++p) {
+                                const int4 sh = tab[cc + p];
+                                const int L = rr[4 * p + 2] * 128 + rr[4 * p + 3];
+                                const int A = (int)((uint32_t)(rr[4 * p] * 128 + rr[4 * p + 1])
+                                                    << sh.y);
+                                const int odd = (A + (L >> sh.x)) & sh.w;
+                                store(p, A + ((L + sh.z + odd) >> sh.x));
+                            }
+                        } else {
+#pragma unroll
+                            for (int p = 0; p < 8; ++p) {
+                                const int r = tab[cc + p].x;
+                                const long long T =
+                                    (((long long)rr[4 * p] * 128 + rr[4 * p + 1]) * 128 +
+                                     rr[4 * p + 2]) * 128 + rr[4 * p + 3];
+                                long long R;
+                                if (r <= 0) R = T << -r;
+                                else R = (T + ((1LL << (r - 1)) - 1) + ((T >> r) & 1)) >> r;
+                                store(p, (int)R);
                             }
                         }
                     }
@@ -363,7 +462,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                             (((long long)rr[4 * p] * 128 + rr[4 * p + 1]) * 128 + rr[4 * p + 2]) *
                                 128 + rr[4 * p + 3];
                         const double sc = __shfl_sync(0xffffffffu, vl < 32 ? scA : scB, vl & 31);
-                        a.Y[((int64_t)k * a.V + v) * a.N_pad + i] = sc * (double)T;
+                        double* const y = a.Y + ((int64_t)k * a.V + v) * a.N_pad + i;
+                        if (a.nsplit > 1) atomicAdd(y, sc * (double)T);
+                        else *y = sc * (double)T;
                     }
                 }
                 }
@@ -571,23 +672,21 @@ void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* s
     count_launch();
 }
 
-size_t p1_umma_smem_bytes() {
-    return (size_t)p1::kStages * p1::kStageBytes + (size_t)p1::kRing * p1::kRingSlot + 1024 + 256;
-}
+size_t p1_umma_smem_bytes(int box_rows) { return (size_t)p1::Layout(box_rows).bytes() + 1024; }
 
 void prepare_p1_umma() {
     cudaFuncSetAttribute(p1_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)p1_umma_smem_bytes());
+                         p1::kSmemLimit);
 }
 
 void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cudaStream_t st) {
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] { prepare_p1_umma(); });
-    const int spc = a.sb_per_cta > 0 ? a.sb_per_cta : 1;
     P1UArgs b = a;
-    b.sb_per_cta = spc;
-    dim3 grid((unsigned)(N_pad / p1::kBM), (unsigned)((a.K + spc - 1) / spc));
-    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(), st>>>(tmW, b);
+    b.sb_per_cta = std::min(std::max(a.sb_per_cta, 1), p1::kMaxSb);
+    b.nsplit = 1;
+    dim3 grid((unsigned)(N_pad / p1::kBM), (unsigned)((a.K + b.sb_per_cta - 1) / b.sb_per_cta));
+    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(a.box_rows), st>>>(tmW, b);
     count_launch();
 }
 
