@@ -56,8 +56,7 @@ constexpr size_t kSmemBytes = (size_t)bar_off() + 256 + 1024;
 __global__ void __launch_bounds__(kThreads, 1)
     gram_ld_kernel(const __grid_constant__ CUtensorMap tmC, GramArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + bar_off());
     uint64_t* pk_full = bars;                    // [kPk] packed rows landed (TMA)
     uint64_t* pk_empty = pk_full + kPk;          // [kPk] packed rows read by the decoders

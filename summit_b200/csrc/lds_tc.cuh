@@ -1,6 +1,7 @@
 // tcgen05 / TMA / mbarrier helpers shared by the tensor-core kernels
 // (inline PTX for sm_100a).
 #pragma once
+#include <climits>
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -48,8 +49,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 // Bounded wait for the phase with the given parity.  Returns false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
-    const long long limit = wait_limit();
-    for (long long i = 0; i < limit; ++i) {
+    const int limit = (int)min(wait_limit(), (long long)INT_MAX);
+    for (int i = 0; i < limit; ++i) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"

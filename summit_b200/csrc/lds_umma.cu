@@ -81,8 +81,7 @@ struct Layout {
 __global__ void __launch_bounds__(kThreads, 1)
     p2_umma_kernel(const __grid_constant__ CUtensorMap tmA, P2UArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
     const Layout lay(a.box_rows);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off());
     uint64_t* pk_full = bars;                          // [kPkStages]
