@@ -320,6 +320,13 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         const int h = (warp - kEpiWarp0) >> 2;   // which quarter of the column chunks
         const int64_t i = i0 + q * 32 + lane;    // sample row of this thread's accumulator lane
         int4* const tab = shift_tab + (warp - kEpiWarp0) * 16;   // this warp's digit shifts
+        // The digit shift of probe vl of this warp's (at most two) chunks of 8,
+        // loaded one job ahead.
+        auto load_shift = [&](int k, int g) {
+            const int v = g * 64 + 8 * (h + 4 * ((lane >> 3) & 1)) + (lane & 7);
+            return v < a.V ? a.yshift[(int64_t)k * a.V + v] : 0;
+        };
+        int shift_next = a.yq ? load_shift(kb0, 0) : 0;
         int au = 0;
         for (int kq = 0; kq < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); ++kq) {
             const int k = kb0 + kq;
@@ -349,6 +356,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                         *reinterpret_cast<uint4*>(a.Y + ((int64_t)k * a.V + (idx >> 6)) * a.N_pad +
                                                   i0 + (idx & 63) * 2) = make_uint4(0, 0, 0, 0);
                 }
+                if (a.yq && kq + 1 < nsb) shift_next = load_shift(k + 1, 0);
                 continue;
             }
             // (nkt is this super-bin's whole list: the digit form is never split)
@@ -361,9 +369,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                 bool narrow = false;
                 double scA = 0.0, scB = 0.0;
                 if (a.yq) {
-                    const int vl = 8 * (h + 4 * ((lane >> 3) & 1)) + (lane & 7);
-                    const int v = g * 64 + vl;
-                    const int r = v < a.V ? -a.yshift[(int64_t)k * a.V + v] : 0;
+                    const int r = -shift_next;
                     narrow = small_sums && __all_sync(0xffffffffu, r >= 0 && r <= 14);
                     // x = right shift, y = 14 - x, z = half an ulp less one, w = parity mask
                     if (lane < 16)
@@ -384,6 +390,8 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                 const int ncols = min(kAccCols, a.ncolp - g * 256);
                 const uint32_t tbase = tmem + (uint32_t)(b * kAccCols) + ((uint32_t)(q * 32) << 16);
                 if (a.yq) {
+                    if (g + 1 < a.ngroups) shift_next = load_shift(k, g + 1);
+                    else if (kq + 1 < nsb) shift_next = load_shift(k + 1, 0);
                     // Digits straight into phase 2's operand layout, 8 probes (32
                     // digit columns) per TMEM load; the quadrant's four warps take
                     // every fourth chunk.  With y = T 2^(eW-28) and the column
@@ -417,13 +425,11 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                         tmem_wait_ld();
                         const int v0 = g * 64 + (c0 >> 2);          // first probe of the chunk (even)
                         const int nv = a.V - v0;                    // probes left (warp-uniform)
-                        auto store = [&](int p, int R) {
-                            uint32_t w = digits_word(R);
-                            w = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 2), selA);
-                            w = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 1), selB);
-                            if (p < nv)
-                                *reinterpret_cast<uint32_t*>(ydst[p & 1] + (int64_t)(v0 + p) * 512) = w;
-                        };
+                        // All roundings before the first store: a store in between
+                        // would order the next probe's shift-table read behind it
+                        // (they could alias) and with it the probes one by one
+                        // (about 2,400 cycles per chunk).
+                        int R[8];
                         if (narrow) {
 #pragma unroll
                             for (int p = 0; p < 8; ++p) {
@@ -432,7 +438,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                                 const int A = (int)((uint32_t)(rr[4 * p] * 128 + rr[4 * p + 1])
                                                     << sh.y);
                                 const int odd = (A + (L >> sh.x)) & sh.w;
-                                store(p, A + ((L + sh.z + odd) >> sh.x));
+                                R[p] = A + ((L + sh.z + odd) >> sh.x);
                             }
                         } else {
 #pragma unroll
@@ -441,12 +447,24 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                                 const long long T =
                                     (((long long)rr[4 * p] * 128 + rr[4 * p + 1]) * 128 +
                                      rr[4 * p + 2]) * 128 + rr[4 * p + 3];
-                                long long R;
-                                if (r <= 0) R = T << -r;
-                                else R = (T + ((1LL << (r - 1)) - 1) + ((T >> r) & 1)) >> r;
-                                store(p, (int)R);
+                                if (r <= 0) R[p] = (int)(T << -r);
+                                else R[p] = (int)((T + ((1LL << (r - 1)) - 1) + ((T >> r) & 1)) >> r);
                             }
                         }
+                        uint32_t w[8];
+#pragma unroll
+                        for (int p = 0; p < 8; ++p) w[p] = digits_word(R[p]);
+#pragma unroll
+                        for (int p = 0; p < 8; ++p)
+                            w[p] = __byte_perm(w[p], __shfl_xor_sync(0xffffffffu, w[p], 2), selA);
+#pragma unroll
+                        for (int p = 0; p < 8; ++p)
+                            w[p] = __byte_perm(w[p], __shfl_xor_sync(0xffffffffu, w[p], 1), selB);
+#pragma unroll
+                        for (int p = 0; p < 8; ++p)
+                            if (p < nv)
+                                *reinterpret_cast<uint32_t*>(ydst[p & 1] + (int64_t)(v0 + p) * 512) =
+                                    w[p];
                     }
                 } else {
                 for (int c0c = 16 * h; c0c < ncols; c0c += 64) {
