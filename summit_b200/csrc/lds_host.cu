@@ -2010,6 +2010,7 @@ void plan_enqueue_phase1(Context& c, GwPlan& pl, size_t ti, double* y, cudaEvent
         pa.Y = y;
         pa.status = static_cast<unsigned*>(pl.status.p);
         pa.m_pad = P.g.M_pad;
+        pa.lmax = t.lmax;
         umma::launch_p1_umma(t.tmW, pa, P.g.N_pad, c.st);
     } else {
         launch_p1_weights(w, static_cast<double*>(P.d_mean.p), static_cast<double*>(P.d_sdinv.p),
@@ -3353,6 +3354,7 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         pa.codes = P.g.codes + (j0 + a) * P.g.nbp;
         pa.colscale = uw.colscale;
         pa.Y = Y;
+        pa.lmax = lmax;
         pa.status = g.status.as<unsigned>(1);
         ck(cudaMemsetAsync(pa.status, 0, 4, c.st), "memset");
         umma::launch_p1_umma(tmW, pa, Np, c.st);

@@ -119,7 +119,8 @@ struct P1UArgs {
     double* Y = nullptr;                // N_pad x (K*V), column (k*V+v)
     unsigned int* status = nullptr;
     int sb_per_cta = 1;                 // super-bins processed by one CTA (pipeline continues)
-    int nsplit = 1;                     // CTAs that share a super-bin's K-steps (FP64 output only)
+    int nsplit = 1;                     // CTAs that share a super-bin's K-steps (set by the launch)
+    int64_t lmax = 0;                   // longest padded list, for that choice (0: no split)
     // Digit output (windowed estimates): when yq is set the epilogue writes the
     // sketch's 4 int8 digits in phase 2's layout (digit_offset, column
     // k*ncolp + 4v + t of K*ncolp) using the a-priori exponents in ycolscale

@@ -1,0 +1,75 @@
+"""GPU: the launch forms that the estimate's kernels choose by size, each at the
+sizes where its split can go wrong, against the FP64 oracle.
+
+Tolerance: weights and sketch enter as 28-bit values of their column's maximum
+(or, windowed, of its a-priori bound), which holds LD scores to the stated 1e-6."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-6
+
+
+def _rows(n, m, seed):
+    """Packed rows of independent hard calls with 2 % missing."""
+    from summit_b200 import bedfile
+
+    rng = np.random.default_rng(seed)
+    g = rng.binomial(2, rng.uniform(0.1, 0.5, (m, 1)), (m, n)).astype(np.int8)
+    g[rng.random((m, n)) < 0.02] = -9
+    return bedfile.pack_bed_rows(g)
+
+
+# (N, M, K, B): lists of 2,304 and 5,000 members share their K-steps among CTAs
+# (the second with an uneven last part, two column groups and an empty bin);
+# 110,000 samples give sketch columns whose cluster slices do not fit the cache,
+# 30,001 ones that do; 1,100 members take the cluster form of the weight digits.
+@pytest.mark.parametrize("n,m,K,B", [(130, 2304, 1, 3), (257, 5000, 3, 70), (110000, 40, 1, 2),
+                                     (30001, 60, 2, 3), (300, 1100, 1, 130)])
+def test_genome_wide_forms(oracle, n, m, K, B):
+    from summit_b200.session import GwSession
+
+    rows = _rows(n, m, seed=n + m)
+    annot = np.ones((m, K))
+    annot[::3, 1:] = 0.0
+    annot[:, 2:] = 0.0
+    sess = GwSession(rows, n)
+    plan = sess.plan(annot, B, 500, 11)
+    plan.execute()
+    first = plan.results()
+    plan.execute()
+    got = plan.results()
+    np.testing.assert_array_equal(first["ldscore"], got["ldscore"])
+    ref = oracle.gw_ldscore(rows, n, annot, nvecs=B, step=500, seed=11)
+    assert rel_err(got["meansq_accum"], ref["meansq_accum"]) < TOL
+    plan.close()
+    sess.close()
+
+
+# Windowed lists: 9,000 equal members push a column's digit shift past 14 (the
+# 64-bit rounding), 300 keep it inside; 66 and 7 probes leave a second column
+# group and a chunk of 8 probes partly filled.
+@pytest.mark.parametrize("n,sizes,B", [(140, [9000], 7), (200, [300, 1, 700], 66),
+                                       (129, [128, 129, 60], 8)])
+def test_windowed_forms(oracle, n, sizes, B):
+    from summit_b200.session import GwSession, WinPlan, window_seed
+
+    ws = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    m = int(ws[-1])
+    rows = _rows(n, m, seed=m)
+    annot = np.ones((m, 2))
+    annot[::2, 1] = 0.0
+    sess = GwSession(rows, n)
+    plan = WinPlan(sess, annot, ws, B, 250, 5)
+    plan.execute()
+    got = plan.results()["meansq_accum"]
+    for w, (a, e) in enumerate(zip(ws[:-1], ws[1:])):
+        ref = oracle.gw_ldscore(rows, n, annot[a:e], nvecs=B, step=250, seed=window_seed(5, w),
+                                snp0=int(a))
+        assert rel_err(got[a:e], ref["meansq_accum"]) < TOL, f"window {w}"
+    plan.close()
+    sess.close()
