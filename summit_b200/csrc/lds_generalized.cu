@@ -14,6 +14,9 @@ namespace lds {
 
 namespace {
 
+// Annotations whose component sums a thread of the diagonal kernel keeps.
+__host__ __device__ constexpr int diag_annots(int P) { return P >= 16 ? 1 : 16 / P; }
+
 // splitmix64 with the increment applied first (generalized_gxe_variant.py
 // _splitmix64), and the addressable sign of global_probe_sign.
 __device__ __forceinline__ uint64_t splitmix64_step(uint64_t v) {
@@ -35,59 +38,127 @@ __global__ void global_probes_kernel(uint64_t root_state, int64_t v0, int64_t L,
     out[idx] = (splitmix64_step(s) >> 63) ? 1.0 : -1.0;
 }
 
-constexpr int kDiagThreads = 128;
-constexpr int kDiagComp = 16;      // components per thread (registers)
+constexpr int kDiagThreads = 128;   // samples per CTA
+constexpr int kDiagRows = 32;       // SNPs staged at a time
 
 // num[c * N + i] += sum_j a[j, k] kf(p) f_q(i, j) f_r(i, j) for the components
-// c = k * P + p of this CTA's chunk, with the projected contextual features
-// f_q(i, j) = phi_q(i) x_ij - sum_r F(i, r) coef[j, q, r] (pass-2 feature
-// tiles, generalized_gxe_pass2.py:528-562) and x_ij the image's standardized
-// genotype (0 on a missing call).  One thread per sample.
+// c = k * P + p of this CTA's annotations, with the projected contextual
+// features f_q(i, j) = phi_q(i) x_ij - sum_r F(i, r) coef[j, q, r] (pass-2
+// feature tiles, generalized_gxe_pass2.py:528-562) and x_ij the image's
+// standardized genotype (0 on a missing call); pairs p = (q, r) diagonals first,
+// then lexicographic off-diagonals, kf 1 on the diagonal and 2 off it.  One
+// thread per sample.
+//
+// Bound by FP64 issue: about Q (R + 2) + 3 P + 2 K P operations per genotype.
+// The SNPs are split over blockIdx.z (a grid of sample tiles alone left most SMs
+// idle), tiles of 32 SNPs' codes, statistics, coefficients and annotations go
+// through shared memory, and Q is a template argument so that the features and
+// their products stay in registers.  A split's sums go to part[z][c][i], added
+// in order by component_diag_reduce_kernel; a single part adds to num itself.
+// N = 4,000, M = 6,000, Q = R = K = 2: 10.2 ms -> 99 us.
+template <int Q, int RM>
 __global__ void __launch_bounds__(kDiagThreads)
     component_diag_kernel(const uint8_t* __restrict__ codes, int64_t nbp,
                           const double* __restrict__ mean, const double* __restrict__ sdinv,
                           int64_t j0, int64_t L, int64_t N, const double* __restrict__ annot,
-                          int K, const double* __restrict__ basis, int Q,
+                          int K, const double* __restrict__ basis,
                           const double* __restrict__ fixed, int R,
-                          const double* __restrict__ coef, const int* __restrict__ pq,
-                          const int* __restrict__ pr, const double* __restrict__ kf, int P,
-                          double* __restrict__ num) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int c0 = blockIdx.y * kDiagComp;
-    const int C = K * P;
-    if (i >= N) return;
-    double phi[kGenMaxQ], frow[kGenMaxR], acc[kDiagComp];
-    for (int q = 0; q < Q; ++q) phi[q] = basis[(int64_t)q * N + i];
-    for (int r = 0; r < R; ++r) frow[r] = fixed[(int64_t)r * N + i];
+                          const double* __restrict__ coef, int64_t rows_per_part,
+                          double* __restrict__ part, double* __restrict__ num) {
+    constexpr int P = Q * (Q + 1) / 2;
+    constexpr int KC = diag_annots(P);   // annotations per CTA
+    __shared__ uint4 s_codes[kDiagRows * 2];
+    __shared__ double s_mean[kDiagRows], s_sd[kDiagRows];
+    __shared__ double s_annot[kDiagRows * KC];
+    __shared__ double s_coef[RM > 0 ? kDiagRows * Q * RM : 1];
+    const int64_t i0 = (int64_t)blockIdx.x * kDiagThreads, i = i0 + threadIdx.x;
+    const int k0 = blockIdx.y * KC, nk = min(KC, K - k0);
+    const bool live = i < N;
+    double phi[Q], frow[RM > 0 ? RM : 1], acc[KC * P];
 #pragma unroll
-    for (int t = 0; t < kDiagComp; ++t) acc[t] = 0.0;
-    const int shift = 2 * (int)(i & 3);
-    for (int64_t jl = 0; jl < L; ++jl) {
-        const int64_t j = j0 + jl;
-        const uint32_t code = (codes[j * nbp + (i >> 2)] >> shift) & 3u;
-        const double g = (double)((code >> 1) + (code == 3u));
-        const double x = code == 1u ? 0.0 : sdinv[j] * (g - mean[j]);
-        double f[kGenMaxQ];
-        for (int q = 0; q < Q; ++q) {
-            double v = phi[q] * x;
-            const double* cj = coef + (jl * Q + q) * R;
-            for (int r = 0; r < R; ++r) v -= frow[r] * cj[r];
-            f[q] = v;
+    for (int q = 0; q < Q; ++q) phi[q] = live ? basis[(int64_t)q * N + i] : 0.0;
+#pragma unroll
+    for (int r = 0; r < RM; ++r) frow[r] = live && r < R ? fixed[(int64_t)r * N + i] : 0.0;
+#pragma unroll
+    for (int t = 0; t < KC * P; ++t) acc[t] = 0.0;
+    const int64_t r0 = (int64_t)blockIdx.z * rows_per_part, r1 = min(L, r0 + rows_per_part);
+    const int shift = 2 * (int)(threadIdx.x & 3);
+    const uint8_t* row_codes = reinterpret_cast<const uint8_t*>(s_codes) + (threadIdx.x >> 2);
+    for (int64_t jb = r0; jb < r1; jb += kDiagRows) {
+        const int rows = (int)min((int64_t)kDiagRows, r1 - jb);
+        __syncthreads();
+        {
+            // 32 bytes of every row: this CTA's 128 samples (rows are padded to
+            // a multiple of 64 bytes, so both halves are inside the image)
+            const int r = threadIdx.x >> 1, c = threadIdx.x & 1;
+            if (r < rows)
+                s_codes[threadIdx.x] = *reinterpret_cast<const uint4*>(
+                    codes + (j0 + jb + r) * nbp + (i0 >> 2) + 16 * c);
         }
+        if (threadIdx.x < rows) {
+            s_mean[threadIdx.x] = mean[j0 + jb + threadIdx.x];
+            s_sd[threadIdx.x] = sdinv[j0 + jb + threadIdx.x];
+        }
+        for (int t = threadIdx.x; t < rows * KC; t += kDiagThreads) {
+            const int r = t / KC, k = t - r * KC;
+            s_annot[t] = k < nk ? annot[(jb + r) * K + k0 + k] : 0.0;
+        }
+        if (RM > 0)
+            for (int t = threadIdx.x; t < rows * Q * RM; t += kDiagThreads) {
+                const int rq = t / RM, r = t - rq * RM;
+                s_coef[t] = r < R ? coef[(jb * Q + rq) * R + r] : 0.0;
+            }
+        __syncthreads();
+        for (int jl = 0; jl < rows; ++jl) {
+            const uint32_t code = ((uint32_t)row_codes[jl * 32] >> shift) & 3u;
+            const double g = (double)((code >> 1) + (code == 3u));
+            const double x = code == 1u ? 0.0 : s_sd[jl] * (g - s_mean[jl]);
+            double f[Q];
 #pragma unroll
-        for (int t = 0; t < kDiagComp; ++t) {
-            const int c = c0 + t;
-            if (c >= C) break;
-            const int k = c / P, p = c - k * P;
-            const double a = annot[jl * K + k];
-            if (a != 0.0) acc[t] += a * (kf[p] * f[pq[p]] * f[pr[p]]);
+            for (int q = 0; q < Q; ++q) {
+                double v = phi[q] * x;
+                const double* cj = s_coef + (jl * Q + q) * RM;
+#pragma unroll
+                for (int r = 0; r < RM; ++r) v -= frow[r] * cj[r];
+                f[q] = v;
+            }
+            double prod[P];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) prod[q] = f[q] * f[q];
+            int p = Q;
+#pragma unroll
+            for (int q = 0; q < Q - 1; ++q)
+#pragma unroll
+                for (int r = q + 1; r < Q; ++r) prod[p++] = 2.0 * f[q] * f[r];
+#pragma unroll
+            for (int k = 0; k < KC; ++k) {
+                const double a = s_annot[jl * KC + k];
+                if (a == 0.0) continue;   // (the same for every sample)
+#pragma unroll
+                for (int t = 0; t < P; ++t) acc[k * P + t] += a * prod[t];
+            }
         }
     }
+    if (!live) return;
 #pragma unroll
-    for (int t = 0; t < kDiagComp; ++t) {
-        const int c = c0 + t;
-        if (c < C) num[(int64_t)c * N + i] += acc[t];
-    }
+    for (int k = 0; k < KC; ++k)
+        if (k < nk)
+#pragma unroll
+            for (int t = 0; t < P; ++t) {
+                const int64_t o = (int64_t)((k0 + k) * P + t) * N + i;
+                if (gridDim.z > 1) part[(int64_t)blockIdx.z * K * P * N + o] = acc[k * P + t];
+                else num[o] += acc[k * P + t];
+            }
+}
+
+// num[o] += the parts' sums in order.
+__global__ void component_diag_reduce_kernel(const double* __restrict__ part, int nparts, int64_t n,
+                                             double* __restrict__ num) {
+    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= n) return;
+    double s = 0.0;
+    for (int z = 0; z < nparts; ++z) s += part[(int64_t)z * n + o];
+    num[o] += s;
 }
 
 // Pass-2 scores of one variant block, one CTA per variant row jl: the row's
@@ -127,18 +198,35 @@ __global__ void gen_rows_kernel(const long long* __restrict__ raw_g,
     }
 }
 
-// directed[c1][c2] += sum_jl a[j0 + jl][k1] rows[jl][p1][c2], c1 = k1 P + p1.
+// directed[c1][c2] += sum_jl a[j0 + jl][k1] rows[jl][p1][c2], c1 = k1 P + p1,
+// in two steps: sums over chunks of kDirRows variants (one CTA each), then one
+// warp per entry over the chunks, both in a fixed order.  One thread per entry
+// over all variants left the chip idle: C = 6, 6,000 variants 786 -> 25 us.
+constexpr int kDirRows = 64;
+
 __global__ void gen_directed_kernel(const double* __restrict__ rows, int64_t L,
                                     const double* __restrict__ annot, int64_t j0, int K, int P,
-                                    double* __restrict__ directed) {
+                                    double* __restrict__ part) {
     const int C = K * P;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= C * C) return;
-    const int c1 = idx / C, c2 = idx - c1 * C, k1 = c1 / P, p1 = c1 - k1 * P;
+    const int64_t r0 = (int64_t)blockIdx.x * kDirRows, r1 = min(L, r0 + kDirRows);
+    for (int idx = threadIdx.x; idx < C * C; idx += blockDim.x) {
+        const int c1 = idx / C, c2 = idx - c1 * C, k1 = c1 / P, p1 = c1 - k1 * P;
+        double s = 0.0;
+#pragma unroll 8
+        for (int64_t jl = r0; jl < r1; ++jl)
+            s += annot[(j0 + jl) * K + k1] * rows[(jl * P + p1) * C + c2];
+        part[(int64_t)blockIdx.x * C * C + idx] = s;
+    }
+}
+
+__global__ void gen_directed_reduce_kernel(const double* __restrict__ part, int64_t nchunks, int n,
+                                           double* __restrict__ directed) {
+    const int idx = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (idx >= n) return;
     double s = 0.0;
-    for (int64_t jl = 0; jl < L; ++jl)
-        s += annot[(j0 + jl) * K + k1] * rows[(jl * P + p1) * C + c2];
-    directed[idx] += s;
+    for (int64_t z = lane; z < nchunks; z += 32) s += part[z * n + idx];
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) directed[idx] += s;
 }
 
 // Pass 2's right-hand side from the contextual sources
@@ -278,12 +366,19 @@ void launch_gen_rows(const long long* raw_g, const long long* raw_o, int64_t raw
     count_launch();
 }
 
+int64_t gen_directed_part_elems(int64_t L, int K, int P) {
+    return (L + kDirRows - 1) / kDirRows * K * P * K * P;
+}
+
 void launch_gen_directed(const double* rows, int64_t L, const double* annot, int64_t j0, int K,
-                         int P, double* directed, cudaStream_t st) {
+                         int P, double* part, double* directed, cudaStream_t st) {
     const int C = K * P;
     if (L <= 0 || C <= 0) return;
-    gen_directed_kernel<<<(unsigned)((C * C + 255) / 256), 256, 0, st>>>(rows, L, annot, j0, K, P,
-                                                                          directed);
+    const int64_t chunks = (L + kDirRows - 1) / kDirRows;
+    gen_directed_kernel<<<(unsigned)chunks, 256, 0, st>>>(rows, L, annot, j0, K, P, part);
+    count_launch();
+    gen_directed_reduce_kernel<<<(unsigned)((C * C + 7) / 8), 256, 0, st>>>(part, chunks, C * C,
+                                                                           directed);
     count_launch();
 }
 
@@ -296,19 +391,59 @@ void launch_global_probes(uint64_t root_state, int64_t v0, int64_t L, int64_t p0
     count_launch();
 }
 
+// SNP parts of a component-diagonal launch: enough CTAs for six per SM, at
+// least one staged tile each, and at most 256 MB of partial sums.
+int component_diag_parts(int64_t N, int64_t L, int K, int Q) {
+    const int P = Q * (Q + 1) / 2;
+    const int64_t ctas = (N + kDiagThreads - 1) / kDiagThreads *
+                         ((K + diag_annots(P) - 1) / diag_annots(P));
+    const int64_t want = (148 * 6 + ctas - 1) / std::max<int64_t>(ctas, 1);
+    const int64_t fit = ((int64_t)256 << 20) / (8 * N * K * P);
+    const int64_t parts = std::min(std::min(want, (L + kDiagRows - 1) / kDiagRows), fit);
+    return (int)std::max<int64_t>(parts, 1);
+}
+
+template <int Q, int RM>
+static void diag_launch(const uint8_t* codes, int64_t nbp, const double* mean, const double* sdinv,
+                        int64_t j0, int64_t L, int64_t N, const double* annot, int K,
+                        const double* basis, const double* fixed, int R, const double* coef,
+                        double* part, double* num, cudaStream_t st) {
+    constexpr int P = Q * (Q + 1) / 2;
+    const int parts = component_diag_parts(N, L, K, Q);
+    const int64_t per = ((L + parts - 1) / parts + kDiagRows - 1) / kDiagRows * kDiagRows;
+    const int used = (int)((L + per - 1) / per);
+    dim3 grid((unsigned)((N + kDiagThreads - 1) / kDiagThreads),
+              (unsigned)((K + diag_annots(P) - 1) / diag_annots(P)), (unsigned)used);
+    component_diag_kernel<Q, RM><<<grid, kDiagThreads, 0, st>>>(
+        codes, nbp, mean, sdinv, j0, L, N, annot, K, basis, fixed, R, coef, per, part, num);
+    count_launch();
+    if (used > 1) {
+        const int64_t n = (int64_t)K * P * N;
+        component_diag_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, used, n, num);
+        count_launch();
+    }
+}
+
+template <int Q>
+static void diag_launch_r(const uint8_t* codes, int64_t nbp, const double* mean,
+                          const double* sdinv, int64_t j0, int64_t L, int64_t N,
+                          const double* annot, int K, const double* basis, const double* fixed,
+                          int R, const double* coef, double* part, double* num, cudaStream_t st) {
+    static_assert(kGenMaxR == 16, "the widest instance holds every fixed effect");
+    auto f = R == 0 ? diag_launch<Q, 0> : R <= 4 ? diag_launch<Q, 4> : diag_launch<Q, 16>;
+    f(codes, nbp, mean, sdinv, j0, L, N, annot, K, basis, fixed, R, coef, part, num, st);
+}
+
 void launch_component_diag(const uint8_t* codes, int64_t nbp, const double* mean,
                            const double* sdinv, int64_t j0, int64_t L, int64_t N,
                            const double* annot, int K, const double* basis, int Q,
-                           const double* fixed, int R, const double* coef, const int* pq,
-                           const int* pr, const double* kf, int P, double* num, cudaStream_t st) {
-    const int C = K * P;
-    if (N <= 0 || L <= 0 || C <= 0) return;
-    dim3 grid((unsigned)((N + kDiagThreads - 1) / kDiagThreads),
-              (unsigned)((C + kDiagComp - 1) / kDiagComp));
-    component_diag_kernel<<<grid, kDiagThreads, 0, st>>>(codes, nbp, mean, sdinv, j0, L, N, annot,
-                                                         K, basis, Q, fixed, R, coef, pq, pr, kf,
-                                                         P, num);
-    count_launch();
+                           const double* fixed, int R, const double* coef, double* part,
+                           double* num, cudaStream_t st) {
+    if (N <= 0 || L <= 0 || K <= 0) return;
+    static_assert(kGenMaxQ == 6, "one instance per basis count");
+    auto f = Q == 1 ? diag_launch_r<1> : Q == 2 ? diag_launch_r<2> : Q == 3 ? diag_launch_r<3>
+           : Q == 4 ? diag_launch_r<4> : Q == 5 ? diag_launch_r<5> : diag_launch_r<6>;
+    f(codes, nbp, mean, sdinv, j0, L, N, annot, K, basis, fixed, R, coef, part, num, st);
 }
 
 }  // namespace lds

@@ -5485,22 +5485,14 @@ LDS_API int lds_generalized_component_diagonal(int64_t geno, int64_t j0, int64_t
                  kGenMaxQ, kGenMaxR);
         Prepared& P = product_image(geno, j0, j1, 1);
         const int64_t L = j1 - j0, N = P.g.N;
-        // pairs: diagonals first, then lexicographic off-diagonals; kernel
-        // factor 1 on the diagonal, 2 off it (context/spec.py ContextPairIndex)
-        std::vector<int> pq, pr;
-        std::vector<double> kf;
-        for (int q = 0; q < Q; ++q) { pq.push_back(q); pr.push_back(q); kf.push_back(1.0); }
-        for (int q = 0; q < Q - 1; ++q)
-            for (int r = q + 1; r < Q; ++r) { pq.push_back(q); pr.push_back(r); kf.push_back(2.0); }
-        const int Pn = (int)pq.size(), C = K * Pn;
-        DevBuf da, db, df, dc, dq, dr, dk, dn;
+        const int C = K * (Q * (Q + 1) / 2);   // components
+        DevBuf da, db, df, dc, dp, dn;
         double* a = da.as<double>((size_t)(L * K));
         double* b = db.as<double>((size_t)(N * Q));
         double* f = df.as<double>((size_t)std::max<int64_t>(N * R, 1));
         double* cf = dc.as<double>((size_t)std::max<int64_t>(L * Q * R, 1));
-        int* qd = dq.as<int>((size_t)Pn);
-        int* rd = dr.as<int>((size_t)Pn);
-        double* kd = dk.as<double>((size_t)Pn);
+        const int parts = component_diag_parts(N, L, K, Q);
+        double* pt = parts > 1 ? dp.as<double>((size_t)parts * (size_t)(C * N)) : nullptr;
         double* nm = dn.as<double>((size_t)(C * N));
         h2d(a, annot, (size_t)(L * K), c.st);
         h2d(b, basis, (size_t)(N * Q), c.st);
@@ -5508,13 +5500,10 @@ LDS_API int lds_generalized_component_diagonal(int64_t geno, int64_t j0, int64_t
             h2d(f, fixed, (size_t)(N * R), c.st);
             h2d(cf, coef, (size_t)(L * Q * R), c.st);
         }
-        h2d(qd, pq.data(), pq.size(), c.st);
-        h2d(rd, pr.data(), pr.size(), c.st);
-        h2d(kd, kf.data(), kf.size(), c.st);
         h2d(nm, numerator, (size_t)(C * N), c.st);
         launch_component_diag(P.g.codes, P.g.nbp, static_cast<double*>(P.d_mean.p),
                               static_cast<double*>(P.d_sdinv.p), j0, L, N, a, K, b, Q, f, R, cf,
-                              qd, rd, kd, Pn, nm, c.st);
+                              pt, nm, c.st);
         ck(cudaGetLastError(), "launch");
         d2h(numerator, nm, (size_t)(C * N), c.st);
         ck(cudaStreamSynchronize(c.st), "component diagonal");
@@ -5551,7 +5540,7 @@ static void gen_pass2_run(Context& c, int64_t geno,
         constexpr int kV2 = 64;
         const int K2 = (cols + kV2 - 1) / kV2, nc = umma::ncolp_for(kV2);
         const int64_t ld = (int64_t)K2 * kV2;
-        DevBuf dY, dyq, dcs, dann, dto, df1, df2, ddir, drg, dro, drows, dst;
+        DevBuf dY, dyq, dcs, dann, dto, df1, df2, ddir, drg, dro, drows, dpart, dst;
         double* Y = dY.as<double>((size_t)(Np * ld));
         ck(cudaMemsetAsync(Y, 0, sizeof(double) * (size_t)(Np * ld), c.st), "memset");
         fill(Y, N, Np);
@@ -5575,6 +5564,7 @@ static void gen_pass2_run(Context& c, int64_t geno,
         long long* rg = drg.as<long long>((size_t)(Lmax * ld));
         long long* ro = dro.as<long long>((size_t)(Lmax * ld));
         double* rows = drows.as<double>((size_t)(Lmax * P * Cc));
+        double* part = dpart.as<double>((size_t)gen_directed_part_elems(Lmax, K, P));
         const CUtensorMap tA = make_map_2d(img.g.codes, (uint64_t)img.g.nbp, (uint64_t)img.g.M_pad,
                                            (uint64_t)img.g.nbp, 32, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
         for (int64_t j0 = 0; j0 < M; j0 += Lmax) {
@@ -5603,7 +5593,7 @@ static void gen_pass2_run(Context& c, int64_t geno,
             launch_gen_rows(rg, ro, ld, cs, static_cast<double*>(img.d_mean.p),
                             static_cast<double*>(img.d_sdinv.p), j0, L, 1.0 / residual_rank, K, B, F,
                             P, to, f1, f2, rows, c.st);
-            launch_gen_directed(rows, L, ann, j0, K, P, dd, c.st);
+            launch_gen_directed(rows, L, ann, j0, K, P, part, dd, c.st);
             ck(cudaGetLastError(), "launch");
             d2h(directional + j0 * P * Cc, rows, (size_t)(L * P * Cc), c.st);
         }

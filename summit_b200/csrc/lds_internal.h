@@ -192,13 +192,17 @@ void launch_gen_rows(const long long* raw_g, const long long* raw_o, int64_t raw
                      const double* cs, const double* mean, const double* sdinv, int64_t j0,
                      int64_t L, double inv_rr, int K, int B, int F, int P, const int* term_off,
                      const int* term_f1, const int* term_f2, double* out, cudaStream_t st);
+// `part`: gen_directed_part_elems doubles of scratch.
+int64_t gen_directed_part_elems(int64_t L, int K, int P);
 void launch_gen_directed(const double* rows, int64_t L, const double* annot, int64_t j0, int K,
-                         int P, double* directed, cudaStream_t st);
+                         int P, double* part, double* directed, cudaStream_t st);
+// `part`: component_diag_parts * K * Q (Q + 1) / 2 * N doubles of scratch (unused with one part).
+int component_diag_parts(int64_t N, int64_t L, int K, int Q);
 void launch_component_diag(const uint8_t* codes, int64_t nbp, const double* mean,
                            const double* sdinv, int64_t j0, int64_t L, int64_t N,
                            const double* annot, int K, const double* basis, int Q,
-                           const double* fixed, int R, const double* coef, const int* pq,
-                           const int* pr, const double* kf, int P, double* num, cudaStream_t st);
+                           const double* fixed, int R, const double* coef, double* part,
+                           double* num, cudaStream_t st);
 
 // Phase-2 product checksums (lds_check.cu): u[wl][i] over the n_windows
 // windows of a batch (K super-bins each, V probes from global probe v0), and

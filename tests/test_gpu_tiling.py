@@ -73,3 +73,30 @@ def test_windowed_forms(oracle, n, sizes, B):
         assert rel_err(got[a:e], ref["meansq_accum"]) < TOL, f"window {w}"
     plan.close()
     sess.close()
+
+
+# One instance per basis count and per range of fixed effects; several
+# annotation chunks, SNP parts of uneven length, a last sample tile of 44.
+@pytest.mark.parametrize("Q,R,K,m", [(1, 0, 20, 70), (2, 2, 6, 33), (3, 5, 3, 200), (4, 4, 2, 31),
+                                     (5, 0, 1, 64), (6, 16, 2, 40)])
+def test_component_diagonal_forms(oracle, Q, R, K, m):
+    from oracle import generalized_oracle as go
+    from summit_b200 import generalized_gxe as gg
+    from summit_b200.session import GwSession
+
+    n = 300
+    rng = np.random.default_rng(Q * 100 + R)
+    rows = _rows(n, m, seed=Q)
+    X = oracle.standardize(rows, n, 0, m)[0]
+    sess = GwSession(rows, n)
+    basis = np.asfortranarray(rng.normal(size=(n, Q)))
+    fixed = np.asfortranarray(np.linalg.qr(rng.normal(size=(n, max(R, 1))))[0][:, :R])
+    annot = rng.random((m, K))
+    annot[::4, 0] = 0.0
+    coef = np.ascontiguousarray(rng.normal(size=(m, Q, R))) if R else None
+    got = rng.normal(size=(K * Q * (Q + 1) // 2, n))
+    want = got.copy()
+    gg._component_diagonal(sess, 0, m, annot, basis, fixed, coef, got)
+    go.component_diagonal(X, 0, m, annot, basis, fixed, coef, want)
+    assert rel_err(got, want) < 1e-12   # FP64 sums of at most 200 terms
+    sess.close()
