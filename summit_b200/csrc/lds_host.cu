@@ -3165,7 +3165,7 @@ struct GxeCtx {
     DevBuf env, common, dirs_ones, ranks_d, ones_M;
     std::vector<DevBuf> basis0;          // per environment: N x rank fixed-effect basis
     // workspaces (grow-only)
-    DevBuf probes, annot, sx, sw, panel, y, wq, wcs, rowind, sc, binoff, coef, coef2, denom;
+    DevBuf probes, annot, sx, sw, panel, y, wq, wcs, rowind, sc, binoff, coef, coef2, denom, leak;
     DevBuf sacc, acc4, guards, status, flag;
     DevBuf dgeno, dw, ones_L;            // dense-block path
     // Exact checks of the target's phase-2 products (lds_gxe_set_checks):
@@ -3394,39 +3394,50 @@ void gxe_project_impl(Context& c, GxeCtx& g, double* panel, int64_t cols, int cp
     }
     // direction and mean from the same values: basis [d_e, 1]
     const int64_t seg = 2 * (int64_t)cpe;
-    double* coef2 = g.coef2.as<double>((size_t)(seg * 2));
+    double* coef2 = g.coef2.as<double>((size_t)(cols * 2));
+    const double* D = static_cast<const double*>(g.dirs_ones.p) + (int64_t)env_start * 2 * N;
+    launch_col_dots(dp, N, N, cols, D, N, 2, 0, coef2, c.st, seg, 2 * N);
+    launch_sub_lowrank(dp, N, N, cols, D, N, 2, coef2, 1, 1.0 / (double)N, c.st, seg, 2 * N);
+    // leakage onto each environment's fixed-effect basis: all environments'
+    // products, then one copy to the host
+    double* dd = g.denom.as<double>((size_t)cols);
+    launch_col_dots(dp, N, N, cols, nullptr, N, 1, 1, dd, c.st);
+    int64_t ranks = 0;
+    for (int64_t e = 0; e < T; ++e) ranks += g.ranks[(size_t)(env_start + e)];
+    double* lc = g.leak.as<double>((size_t)std::max<int64_t>(seg * ranks, 1));
+    std::vector<double> den((size_t)cols), co((size_t)(seg * ranks));
+    int64_t at = 0;
     for (int64_t e = 0; e < T; ++e) {
-        double* v = dp + e * seg * N;
-        const double* D = static_cast<const double*>(g.dirs_ones.p) + (env_start + e) * 2 * N;
-        launch_col_dots(v, N, N, seg, D, N, 2, 0, coef2, c.st);
-        launch_sub_lowrank(v, N, N, seg, D, N, 2, coef2, 1, 1.0 / (double)N, c.st);
-    }
-    // leakage onto each environment's fixed-effect basis
-    std::vector<double> den((size_t)seg), co;
-    for (int64_t e = 0; e < T; ++e) {
-        const int env = (int)(env_start + e);
-        const int rank = g.ranks[(size_t)env];
-        double* v = dp + e * seg * N;
-        double* dd = g.denom.as<double>((size_t)seg);
-        launch_col_dots(v, N, N, seg, nullptr, N, 1, 1, dd, c.st);
-        std::vector<double> leaked((size_t)seg, 0.0);
-        d2h(den.data(), dd, (size_t)seg, c.st);
+        const int env = (int)(env_start + e), rank = g.ranks[(size_t)env];
         for (int a0 = 0; a0 < rank; a0 += mb) {
             const int nb = std::min(mb, rank - a0);
-            double* coef = g.coef.as<double>((size_t)(seg * nb));
             const double* B0 = static_cast<const double*>(g.basis0[(size_t)env].p) + (int64_t)a0 * N;
-            launch_col_dots(v, N, N, seg, B0, N, nb, 0, coef, c.st);
-            co.resize((size_t)(seg * nb));
-            d2h(co.data(), coef, co.size(), c.st);
-            ck(cudaStreamSynchronize(c.st), "gxe leakage");
-            for (int64_t q = 0; q < seg; ++q)
-                for (int a = 0; a < nb; ++a) leaked[(size_t)q] += co[(size_t)(q * nb + a)] * co[(size_t)(q * nb + a)];
+            launch_col_dots(dp + e * seg * N, N, N, seg, B0, N, nb, 0, lc + at, c.st);
+            at += seg * nb;
         }
-        ck(cudaStreamSynchronize(c.st), "gxe leakage");
+    }
+    ck(cudaGetLastError(), "launch");
+    d2h(den.data(), dd, den.size(), c.st);
+    d2h(co.data(), lc, co.size(), c.st);
+    ck(cudaStreamSynchronize(c.st), "gxe leakage");
+    at = 0;
+    for (int64_t e = 0; e < T; ++e) {
+        const int rank = g.ranks[(size_t)(env_start + e)];
+        std::vector<double> leaked((size_t)seg, 0.0);
+        for (int a0 = 0; a0 < rank; a0 += mb) {
+            const int nb = std::min(mb, rank - a0);
+            for (int64_t q = 0; q < seg; ++q)
+                for (int a = 0; a < nb; ++a) {
+                    const double x = co[(size_t)(at + q * nb + a)];
+                    leaked[(size_t)q] += x * x;
+                }
+            at += seg * nb;
+        }
         double maximum = 0.0;
         for (int64_t q = 0; q < seg; ++q) {
-            const double rel = den[(size_t)q] > 0.0 ? std::sqrt(leaked[(size_t)q] / den[(size_t)q])
-                                                    : std::numeric_limits<double>::infinity();
+            const double d = den[(size_t)(e * seg + q)];
+            const double rel = d > 0.0 ? std::sqrt(leaked[(size_t)q] / d)
+                                       : std::numeric_limits<double>::infinity();
             if (!std::isfinite(rel)) fail(LDS_ERR_ARG, "Multi-environment native source leakage is non-finite");
             maximum = std::max(maximum, rel);
         }

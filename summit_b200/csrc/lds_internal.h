@@ -134,14 +134,16 @@ void launch_gxe_source_finalize(const double* Y, int64_t N, int64_t N_pad, int64
                                 int64_t t_ld, cudaStream_t st);
 // out[c nb + a] = basis_a . panel_c (basis null: column sums, nb = 1); with
 // `squares` out[c] = panel_c . panel_c.  nb <= col_dots_max_basis().
+// (columns [g group_cols, (g + 1) group_cols) use the basis at basis + g group_stride)
 void launch_col_dots(const double* panel, int64_t p_ld, int64_t N, int64_t C, const double* basis,
-                     int64_t b_ld, int nb, int squares, double* out, cudaStream_t st);
+                     int64_t b_ld, int nb, int squares, double* out, cudaStream_t st,
+                     int64_t group_cols = 0, int64_t group_stride = 0);
 int col_dots_max_basis();
 // panel_c -= sum_a basis_a coef[c nb + a] (the last basis column is all ones,
 // scaled by last_scale, when ones_last).
 void launch_sub_lowrank(double* panel, int64_t ld, int64_t N, int64_t C, const double* basis,
                         int64_t b_ld, int nb, const double* coef, int ones_last, double last_scale,
-                        cudaStream_t st);
+                        cudaStream_t st, int64_t group_cols = 0, int64_t group_stride = 0);
 void launch_gxe_pair(const double* S, int64_t s_ld, int64_t N, int64_t N_pad, int64_t C,
                      int64_t cols_per_group, const double* w, int64_t w_ld, int w_first,
                      double* Ypair, cudaStream_t st);
