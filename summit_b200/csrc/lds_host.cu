@@ -3355,6 +3355,14 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         pa.colscale = uw.colscale;
         pa.Y = Y;
         pa.lmax = lmax;
+        // With one annotation bin every (environment, half) has the same member
+        // list (they differ in the scales), so as many as fill 256 digit columns
+        // share each gathered and decoded genotype tile.  E = 4, B = 32, N = M =
+        // 20,000: source products 1.00 -> 0.77 ms.
+        if (K == 1 && nc <= 128) {
+            pa.share = (int)std::min<int64_t>(G, 256 / nc);
+            pa.sb_per_cta = pa.share;
+        }
         pa.status = g.status.as<unsigned>(1);
         ck(cudaMemsetAsync(pa.status, 0, 4, c.st), "memset");
         umma::launch_p1_umma(tmW, pa, Np, c.st);

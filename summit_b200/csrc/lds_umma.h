@@ -119,6 +119,9 @@ struct P1UArgs {
     double* Y = nullptr;                // N_pad x (K*V), column (k*V+v)
     unsigned int* status = nullptr;
     int sb_per_cta = 1;                 // super-bins processed by one CTA (pipeline continues)
+    // Consecutive super-bins with identical member lists whose columns one job
+    // takes side by side: share * ncolp <= 256, FP64 output, ngroups 1.
+    int share = 1;
     int nsplit = 1;                     // CTAs that share a super-bin's K-steps (set by the launch)
     int64_t lmax = 0;                   // longest padded list, for that choice (0: no split)
     // Digit output (windowed estimates): when yq is set the epilogue writes the
@@ -130,6 +133,11 @@ struct P1UArgs {
     const int* yshift = nullptr;        // K*V digit shifts eW - eY (from the weight kernel)
     int64_t m_pad = 0;                  // image rows, for the bounds-checked build (0: unchecked)
 };
+
+// Rows of a weight-digit tile in shared memory.
+__host__ __device__ inline int p1_tile_rows(const P1UArgs& a) {
+    return a.share > 1 ? a.share * a.ncolp : a.box_rows;
+}
 
 struct P1UWeights {
     int K = 0, V = 0, ncolp = 0;
@@ -145,7 +153,7 @@ struct P1UWeights {
 
 void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* sdinv,
                         const double* Z, int64_t z_ld, cudaStream_t st);
-size_t p1_umma_smem_bytes(int box_rows);
+size_t p1_umma_smem_bytes(int tile_rows);
 void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cudaStream_t st);
 
 // Columns per bin (4 digits per probe, padded to a multiple of 16).

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     using namespace p1;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
-    const Layout lay(a.box_rows);
+    const Layout lay(p1_tile_rows(a));
     const int nst = lay.stages;
     uint8_t* ring = smem + lay.ring_off();
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off());
@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t i0 = (int64_t)blockIdx.x * kBM;
     // This CTA's super-bins: kb0 .. kb0 + nsb; a job is one (super-bin, column
-    // group).  ktab holds their list offsets in K-steps.  With nsplit > 1 the CTA
+    // group), or with share > 1 that many super-bins with one member list, their
+    // digit columns side by side, so that a decoded tile serves them all.  ktab holds their list offsets in K-steps.  With nsplit > 1 the CTA
     // takes part blockIdx.z of every super-bin's K-steps.
     const int kb0 = blockIdx.y * a.sb_per_cta;
     const int nsb = min(a.K - kb0, a.sb_per_cta);
@@ -155,18 +156,21 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         if (lane == 0) {
             int it = 0, s = 0;
             uint32_t ph = 0;
-            for (int q = 0; q < nsb && !*abort_flag; ++q) {
+            for (int q = 0; q < nsb && !*abort_flag; q += a.share) {
                 int k0;
-                const int nkt = steps_of(q, k0);
+                const int nkt = steps_of(q, k0), nbin = min(a.share, nsb - q);
                 for (int g = 0; g < a.ngroups && !*abort_flag; ++g) {
                     for (int kt = 0; kt < nkt; ++kt, ++it) {
                         if (it >= nst && !mbar_wait(&empty[s], ph ^ 1u)) { fail(11); break; }
                         if (*abort_flag) break;
                         uint8_t* w = smem + s * lay.stage + 2 * kATile;
-                        mbar_expect_tx(&full_w[s], (uint32_t)(2 * a.box_rows * kBK));
-                        const int y0 = (kb0 + q) * 2 * a.ncolp + g * 256;
-                        tma_load_2d(w, &tmW, (k0 + kt) * kBK, y0, &full_w[s]);
-                        tma_load_2d(w + lay.w_tile, &tmW, (k0 + kt) * kBK, y0 + a.ncolp, &full_w[s]);
+                        mbar_expect_tx(&full_w[s], (uint32_t)(2 * nbin * a.box_rows * kBK));
+                        for (int u = 0; u < nbin; ++u, w += a.ncolp * kBK) {
+                            const int y0 = (kb0 + q + u) * 2 * a.ncolp + g * 256;
+                            tma_load_2d(w, &tmW, (k0 + kt) * kBK, y0, &full_w[s]);
+                            tma_load_2d(w + lay.w_tile, &tmW, (k0 + kt) * kBK, y0 + a.ncolp,
+                                        &full_w[s]);
+                        }
                         if (++s == nst) { s = 0; ph ^= 1u; }
                     }
                 }
@@ -181,13 +185,14 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         if (lane == 0) {
             int s = 0, au = 0;  // stage, jobs (accumulator uses)
             uint32_t ph = 0;
-            for (int q = 0; q < nsb && !*abort_flag; ++q) {
+            for (int q = 0; q < nsb && !*abort_flag; q += a.share) {
                 int k0;
                 const int nkt = steps_of(q, k0);
+                const int width = min(a.share, nsb - q) * a.ncolp;   // the job's digit columns
                 if (nkt == 0) continue;
                 for (int g = 0; g < a.ngroups && !*abort_flag; ++g, ++au) {
                     const int b = au & 1, u = au >> 1;
-                    const int ncols = min(kAccCols, a.ncolp - g * 256);
+                    const int ncols = min(kAccCols, width - g * 256);
                     const uint32_t idesc = idesc_i8_amn(kBM, ncols);
                     const uint32_t acc = tmem + (uint32_t)(b * kAccCols);
                     if (u > 0 && !mbar_wait(&acc_empty[b], (uint32_t)(u - 1) & 1u)) { fail(12); break; }
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         // read from rowind one step earlier (row_next), so that load's latency
         // overlaps a step of work instead of stalling the cp.async that needs
         // the address.
-        int pq = -1, pg = a.ngroups - 1, pkt = 0, pn = 0, pit = 0;
+        int pq = -a.share, pg = a.ngroups - 1, pkt = 0, pn = 0, pit = 0;
         const int32_t* prow = nullptr;
         bool pend = false;
         auto advance = [&]() {   // cursor to the next K-step, or pend past the last one
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             pg = 0;
             int k0 = 0;
             do {
-                if (++pq >= nsb) {
+                if ((pq += a.share) >= nsb) {
                     pend = true;
                     return;
                 }
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         for (int d = 0; d < kDepth - 1; ++d) prefetch_one();
         int it = 0, s = 0, slot = 0;
         uint32_t ph = 0;
-        for (int q = 0; q < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); ++q) {
+        for (int q = 0; q < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); q += a.share) {
             int k0;
             const int nkt = steps_of(q, k0) * a.ngroups;
             for (int kt = 0; kt < nkt; ++kt, ++it) {
@@ -326,12 +331,19 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             const int v = g * 64 + 8 * (h + 4 * ((lane >> 3) & 1)) + (lane & 7);
             return v < a.V ? a.yshift[(int64_t)k * a.V + v] : 0;
         };
+        // Sketch column, counted from the job's first bin, of digit-column group
+        // `slot` (4 columns each): -1 past a bin's probes or the job's bins.
+        auto probe_of = [&](int slot, int nbin) -> int64_t {
+            if (a.share == 1) return slot < a.V ? slot : -1;
+            const int per = a.ncolp / 4, u = slot / per, v = slot - u * per;
+            return u < nbin && v < a.V ? (int64_t)u * a.V + v : -1;
+        };
         int shift_next = a.yq ? load_shift(kb0, 0) : 0;
         int au = 0;
-        for (int kq = 0; kq < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); ++kq) {
+        for (int kq = 0; kq < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); kq += a.share) {
             const int k = kb0 + kq;
             int k0;
-            const int nkt = steps_of(kq, k0);
+            const int nkt = steps_of(kq, k0), nbin = min(a.share, nsb - kq);
             // This sample tile's block of super-bin k in phase 2's digit layout
             // (digit_offset): ncolp rows of 128 bytes.
             int8_t* const yblk =
@@ -352,7 +364,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                         *reinterpret_cast<uint4*>(yblk + (idx >> 3) * 128 + (idx & 7) * 16) =
                             make_uint4(0, 0, 0, 0);
                 } else if (a.nsplit <= 1) {
-                    for (int idx = e; idx < a.V * 64; idx += kEpiThreads)
+                    for (int idx = e; idx < nbin * a.V * 64; idx += kEpiThreads)
                         *reinterpret_cast<uint4*>(a.Y + ((int64_t)k * a.V + (idx >> 6)) * a.N_pad +
                                                   i0 + (idx & 63) * 2) = make_uint4(0, 0, 0, 0);
                 }
@@ -377,17 +389,16 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                                               r > 0 ? 1 : 0);
                     __syncwarp();
                 } else {
-                    const int va = g * 64 + lane, vb = va + 32;
-                    const int64_t o = (int64_t)k * a.V;
-                    if (va < a.V) scA = a.colscale[o + va];
-                    if (vb < a.V) scB = a.colscale[o + vb];
+                    const int64_t oa = probe_of(g * 64 + lane, nbin), ob = probe_of(g * 64 + lane + 32, nbin);
+                    if (oa >= 0) scA = a.colscale[(int64_t)k * a.V + oa];
+                    if (ob >= 0) scB = a.colscale[(int64_t)k * a.V + ob];
                 }
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (uint32_t)u & 1u))) {
                     fail(15);
                     break;
                 }
                 tc_fence_after();
-                const int ncols = min(kAccCols, a.ncolp - g * 256);
+                const int ncols = min(kAccCols, nbin * a.ncolp - g * 256);
                 const uint32_t tbase = tmem + (uint32_t)(b * kAccCols) + ((uint32_t)(q * 32) << 16);
                 if (a.yq) {
                     if (g + 1 < a.ngroups) shift_next = load_shift(k, g + 1);
@@ -474,13 +485,13 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
                         const int vl = c0c / 4 + p;  // probe within the group (warp-uniform)
-                        const int v = g * 64 + vl;
-                        if (v >= a.V) continue;
+                        const int64_t o = probe_of(g * 64 + vl, nbin);
+                        if (o < 0) continue;
                         const long long T =
                             (((long long)rr[4 * p] * 128 + rr[4 * p + 1]) * 128 + rr[4 * p + 2]) *
                                 128 + rr[4 * p + 3];
                         const double sc = __shfl_sync(0xffffffffu, vl < 32 ? scA : scB, vl & 31);
-                        double* const y = a.Y + ((int64_t)k * a.V + v) * a.N_pad + i;
+                        double* const y = a.Y + ((int64_t)k * a.V + o) * a.N_pad + i;
                         if (a.nsplit > 1) atomicAdd(y, sc * (double)T);
                         else *y = sc * (double)T;
                     }
@@ -690,7 +701,7 @@ void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* s
     count_launch();
 }
 
-size_t p1_umma_smem_bytes(int box_rows) { return (size_t)p1::Layout(box_rows).bytes() + 1024; }
+size_t p1_umma_smem_bytes(int tile_rows) { return (size_t)p1::Layout(tile_rows).bytes() + 1024; }
 
 void prepare_p1_umma() {
     cudaFuncSetAttribute(p1_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -701,7 +712,8 @@ void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cud
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] { prepare_p1_umma(); });
     P1UArgs b = a;
-    b.sb_per_cta = std::min(std::max(a.sb_per_cta, 1), p1::kMaxSb);
+    b.share = std::max(a.share, 1);   // (whole groups per CTA)
+    b.sb_per_cta = std::max(std::min(a.sb_per_cta, p1::kMaxSb) / b.share, 1) * b.share;
     dim3 grid((unsigned)(N_pad / p1::kBM), (unsigned)((a.K + b.sb_per_cta - 1) / b.sb_per_cta));
     // Few sample tiles leave SMs idle while each CTA walks its whole list: as
     // many CTAs as fill the chip once then share a list's K-steps (8 at least
@@ -716,7 +728,7 @@ void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cud
     grid.z = (unsigned)b.nsplit;
     if (b.nsplit > 1)
         cudaMemsetAsync(a.Y, 0, sizeof(double) * (size_t)(a.K * a.V) * (size_t)N_pad, st);
-    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(a.box_rows), st>>>(tmW, b);
+    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(p1_tile_rows(b)), st>>>(tmW, b);
     count_launch();
 }
 
