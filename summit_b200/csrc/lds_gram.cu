@@ -204,7 +204,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tmem_ld16(tb + 128u + (uint32_t)c0, go);
                     tmem_ld16(tb + 256u + (uint32_t)c0, og);
                     tmem_ld16(tb + 384u + (uint32_t)c0, oo);
-                    tmem_wait_ld();
+                    tmem_wait_ld(gg);
+                    tmem_wait_ld(go);
+                    tmem_wait_ld(og);
+                    tmem_wait_ld(oo);
 #pragma unroll
                     for (int u = 0; u < 16; ++u) {
                         const int64_t i = ib + c0 + u;  // warp-uniform

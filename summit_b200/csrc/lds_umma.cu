@@ -10,14 +10,23 @@
 //   * two sets of 4 decoder warps expanding packed codes into the G (value)
 //     and O (observed) int8 operand tiles in the canonical K-major
 //     SWIZZLE_128B layout the UMMA descriptors expect;
-//   * one thread issuing tcgen05.mma.kind::i8 (M=128, N<=256, K=32) into two
-//     TMEM accumulators (G at column 0, O at column 256; on tiles without a
-//     missing call, two alternating G accumulators);
+//   * a warp issuing tcgen05.mma.kind::i8 (M=128, N<=256, K=32) from one elected
+//     thread into two TMEM accumulators (G at column 0, O at column 256; on tiles
+//     without a missing call, the column groups' G products in turn);
 //   * the first decoder set reading the accumulators back with tcgen05.ld for
 //     the exact digit recombination and the squared-sum epilogue.
 // The CTA's bins' columns are walked in MMA groups of up to 256, a bin
-// possibly straddling two groups: an MMA costs about the same at N = 64 and
-// N = 256, so full groups do the most work per instruction.
+// possibly straddling two groups: the issuing warp's time per K-step is nearly
+// the same at N = 64 and N = 256, so full groups do the most work for it.
+//
+// What bounds it: the int8 tensor pipe (1,076 cycles per K-step of 256 columns,
+// 1,024 of them MMA, at the power-capped clock).  Before the issuing loop was
+// made warp-uniform with one wait and one commit per K-step it took 1,316, and a
+// group's epilogue 38,000 cycles (now 12,000; the reads of its probe table were
+// chained behind the outputs).  N = 50,000, M = 40,000, K = 24, B = 50: 12.6 ->
+// 11.1 ms; windowed, M = 60,000: 19.8 -> 17.5 ms; N = 200,003, K = 1: 1.04 -> 0.84
+// ms; N = 10,007, HWE, K = 6, B = 10: 180 -> 141 us; N = 5,000, M = 20,000,
+// B = 20: 72 -> 53 us.
 // Digits of each probe column sit next to each other (column = 4 v + t), so
 // one 32-column TMEM load holds 8 probes x 4 digits.
 //
@@ -42,40 +51,38 @@ constexpr int kBM = 128;              // SNP rows per CTA (UMMA M)
 constexpr int kBK = 128;              // samples per stage (bytes per operand row)
 constexpr int kPkBytes = kBM * 32;    // packed tile: 128 rows x 32 bytes
 constexpr int kATile = kBM * kBK;     // 16 KB
-#ifndef LDS_P2_PK_STAGES
-#define LDS_P2_PK_STAGES 8
-#endif
-#ifndef LDS_P2_A_STAGES
-#define LDS_P2_A_STAGES 2
-#endif
-#ifndef LDS_P2_B_STAGES
-#define LDS_P2_B_STAGES 4
-#endif
-constexpr int kPkStages = LDS_P2_PK_STAGES;  // packed-code ring (HBM latency)
-constexpr int kAStages = LDS_P2_A_STAGES;    // decoded G/O operand ring
-constexpr int kBStages = LDS_P2_B_STAGES;    // sketch-digit ring (L2 latency)
+constexpr int kPkStages = 6;          // packed-code ring (HBM latency)
+// Operand ring: a stage holds a K-step's decoded G and O tiles and its sketch
+// tile.  The issuing warp waits on one barrier per K-step and commits to one:
+// the first decoder warp of a step waits for the sketch tile before it arrives.
+constexpr int kStages = 3;
 // Decoder sets: set d decodes the K-steps it with it % kDecSets == d, so two
 // sets keep two operand tiles in flight while the first set also runs the
 // epilogue.
-#ifndef LDS_P2_DEC_SETS
-#define LDS_P2_DEC_SETS 2
-#endif
-constexpr int kDecSets = LDS_P2_DEC_SETS;
+constexpr int kDecSets = 2;
 constexpr int kThreads = 96 + 128 * kDecSets;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kOCol = 256;       // TMEM column of the O accumulator
+
+// What an epilogue thread needs of one probe column group (4 digit columns).
+struct __align__(16) ProbeSlot {
+    double scale;          // the sketch column's scale
+    long long colsum;      // recombined digit column sums (tiles without a missing call)
+    int bin;               // bin offset within the CTA's bins, -1: no output uses the columns
+    int v;                 // probe
+};
 
 struct Layout {
     uint32_t b_slot;                  // bytes of one sketch tile (box_rows x 128, 1 KB multiple)
     __host__ __device__ explicit Layout(int box_rows)
         : b_slot((uint32_t)(((box_rows * kBK) + 1023) / 1024 * 1024)) {}
-    __host__ __device__ uint32_t a_off(int s) const { return (uint32_t)s * 2 * kATile; }
-    __host__ __device__ uint32_t b_off(int s) const { return kAStages * 2 * kATile + s * b_slot; }
-    __host__ __device__ uint32_t pk_off(int s) const {
-        return kAStages * 2 * kATile + kBStages * b_slot + s * kPkBytes;
-    }
+    __host__ __device__ uint32_t a_off(int s) const { return (uint32_t)s * (2 * kATile + b_slot); }
+    __host__ __device__ uint32_t b_off(int s) const { return a_off(s) + 2 * kATile; }
+    __host__ __device__ uint32_t pk_off(int s) const { return a_off(kStages) + s * kPkBytes; }
     __host__ __device__ uint32_t bar_off() const { return pk_off(kPkStages); }
-    __host__ __device__ uint32_t bytes() const { return bar_off() + 256; }
+    // 64 probe slots for each of the four epilogue warps
+    __host__ __device__ uint32_t slot_off() const { return bar_off() + 256; }
+    __host__ __device__ uint32_t bytes() const { return slot_off() + 4 * 64 * sizeof(ProbeSlot); }
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -86,16 +93,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off());
     uint64_t* pk_full = bars;                          // [kPkStages]
     uint64_t* pk_empty = pk_full + kPkStages;          // [kPkStages]
-    uint64_t* a_full = pk_empty + kPkStages;           // [kAStages]
-    uint64_t* a_empty = a_full + kAStages;             // [kAStages]
-    uint64_t* b_full = a_empty + kAStages;             // [kBStages]
-    uint64_t* b_empty = b_full + kBStages;             // [kBStages]
-    uint64_t* acc_full = b_empty + kBStages;
-    uint64_t* acc_empty = acc_full + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    uint64_t* b_full = pk_empty + kPkStages;           // [kStages] sketch tile landed
+    uint64_t* full = b_full + kStages;                 // [kStages] operands decoded and landed
+    uint64_t* empty = full + kStages;                  // [kStages] operands consumed
+    uint64_t* acc_full = empty + kStages;              // [2] accumulator holds a finished group
+    uint64_t* acc_empty = acc_full + 2;                // [2] accumulator read out
+    uint64_t* mma_done = acc_empty + 2;                // drain of the issuer's MMAs
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     // This CTA's bins: k0 .. k0 + nbk - 1, sharing each decoded genotype tile;
     // their sketch columns are consecutive (bin-major), one TMA box for all.
     // (tile, bin group) of this CTA: the grid's (x, y), or entry x of the work
@@ -129,16 +136,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(&pk_full[s], 1);
             mbar_init(&pk_empty[s], 4);   // one arrival per decoder warp
         }
-        for (int s = 0; s < kAStages; ++s) {
-            mbar_init(&a_full[s], 4);     // one arrival per decoder warp
-            mbar_init(&a_empty[s], 1);
-        }
-        for (int s = 0; s < kBStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(&b_full[s], 1);
-            mbar_init(&b_empty[s], 1);
+            mbar_init(&full[s], 4);       // one arrival per decoder warp
+            mbar_init(&empty[s], 1);
         }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, 4);          // one arrival per epilogue warp
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 4);  // one arrival per epilogue warp
+        }
+        mbar_init(mma_done, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -152,7 +159,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // A tile whose output rows have no missing call needs no O plane.
+    // A tile whose output rows have no missing call needs no O plane: its groups
+    // take the two accumulators in turn, so that one is read out while the next
+    // group's MMAs fill the other.
     int no_missing = (a.snp_missing && a.colsum) ? 1 : 0;
     if (no_missing && tid < kBM) {
         const int64_t j = jt0 + tid;
@@ -170,16 +179,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int ngroups = min(a.ngroups, (nbk * a.ncolp + 255) / 256);
     const int total = ngroups * a.nkt;
     if (warp == 0) {
-        // ---------------- packed-code producer (runs up to 8 stages ahead) ----------------
+        // ---------------- packed-code producer (runs up to kPkStages ahead) ----------------
         if (lane == 0) {
-            int it = 0;
+            int it = 0, s = 0;
+            uint32_t ph = 0;
             for (; it < total; ++it) {
-                const int s = it % kPkStages;
-                if (it >= kPkStages &&
-                    !mbar_wait(&pk_empty[s], ((uint32_t)(it / kPkStages) & 1u) ^ 1u)) { fail(1); break; }
-                if (*abort_flag) break;
+                if (it >= kPkStages && !mbar_wait(&pk_empty[s], ph ^ 1u, abort_flag)) { fail(1); break; }
                 mbar_expect_tx(&pk_full[s], (uint32_t)kPkBytes);
                 tma_load_2d(smem + lay.pk_off(s), &tmA, (it % a.nkt) * 32, (int)jt0, &pk_full[s]);
+                if (++s == kPkStages) { s = 0; ph ^= 1u; }
             }
             // Drain: no tile copy may still be landing when the CTA exits (only
             // reachable with copies outstanding after an abort).  Each slot's
@@ -190,71 +198,87 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp == 2) {
         // ---------------- sketch-digit producer ----------------
         if (lane == 0) {
-            int it = 0;
-            for (; it < total; ++it) {
-                const int s = it % kBStages;
-                if (it >= kBStages &&
-                    !mbar_wait(&b_empty[s], ((uint32_t)(it / kBStages) & 1u) ^ 1u)) { fail(2); break; }
-                if (*abort_flag) break;
-                const int g = it / a.nkt, kt = it % a.nkt;
+            int it = 0, s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int g = 0; g < ngroups && ok; ++g) {
                 // The group's columns that exist (this CTA's bins); MMA columns
                 // past them read stale rows whose results no output uses.
                 const int live = min(min(256, cols - g * 256), nbk * a.ncolp - g * 256);
                 const uint32_t bytes = (uint32_t)live * (uint32_t)kBK;
-                mbar_expect_tx(&b_full[s], bytes);
-                // two copies of whole 16-row pieces (2 KB multiples): phase 2
-                // measured ~2 % faster than with one copy of up to 32 KB
-                const int8_t* src =
-                    a.yq + ((int64_t)kt * a.yq_cols + (int64_t)kb * a.ncolp + g * 256) * kBK;
                 const uint32_t first = (uint32_t)(live / 32) * 16u * (uint32_t)kBK;
-                if (first) bulk_load(smem + lay.b_off(s), src, first, &b_full[s]);
-                bulk_load(smem + lay.b_off(s) + first, src + first, bytes - first, &b_full[s]);
+                const int8_t* src = a.yq + ((int64_t)kb * a.ncolp + g * 256) * kBK;
+                for (int kt = 0; kt < a.nkt; ++kt, ++it, src += a.yq_cols * kBK) {
+                    if (it >= kStages && !mbar_wait(&empty[s], ph ^ 1u, abort_flag)) {
+                        fail(2);
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&b_full[s], bytes);
+                    // two copies of whole 16-row pieces (2 KB multiples): phase 2
+                    // measured ~2 % faster than with one copy of up to 32 KB
+                    if (first) bulk_load(smem + lay.b_off(s), src, first, &b_full[s]);
+                    bulk_load(smem + lay.b_off(s) + first, src + first, bytes - first, &b_full[s]);
+                    if (++s == kStages) { s = 0; ph ^= 1u; }
+                }
             }
-            for (int j = max(0, it - kBStages); j < it; ++j)
-                mbar_wait(&b_full[j % kBStages], (uint32_t)(j / kBStages) & 1u);
+            for (int j = max(0, it - kStages); j < it; ++j)
+                mbar_wait(&b_full[j % kStages], (uint32_t)(j / kStages) & 1u);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int it = 0;
-            for (int g = 0; g < ngroups && !*abort_flag; ++g) {
-                const int ncols = min(256, cols - g * 256);
-                const uint32_t idesc = idesc_i8(kBM, ncols);
-                if (g > 0 && !mbar_wait(acc_empty, (uint32_t)(g - 1) & 1u)) { fail(3); break; }
+        // The whole warp walks the loop, so that addresses, phases and descriptors
+        // stay in uniform registers, and one elected thread issues: the loop of a
+        // single diverged thread took 1,316 cycles per K-step with its operands
+        // always ready (MMAs 1,024).
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int g = 0; g < ngroups && ok; ++g) {
+            const int b = complete ? g & 1 : 0, u = complete ? g >> 1 : g;
+            const int ncols = min(256, cols - g * 256);
+            const uint32_t idesc = idesc_i8(kBM, ncols);
+            const uint32_t acc = tmem + (uint32_t)b * kOCol;
+            if (u > 0 && !warp_wait(&acc_empty[b], (uint32_t)(u - 1) & 1u, abort_flag)) {
+                fail(3);
+                break;
+            }
+            tc_fence_after();
+            for (int kt = 0; kt < a.nkt; ++kt) {
+                if (!warp_wait(&full[s], ph, abort_flag)) {
+                    fail(4);
+                    ok = false;
+                    break;
+                }
                 tc_fence_after();
-                for (int kt = 0; kt < a.nkt; ++kt, ++it) {
-                    const int sa = it % kAStages, sb = it % kBStages;
-                    if (!mbar_wait(&a_full[sa], (uint32_t)(it / kAStages) & 1u) ||
-                        !mbar_wait(&b_full[sb], (uint32_t)(it / kBStages) & 1u)) { fail(4); break; }
-                    if (*abort_flag) break;
-                    tc_fence_after();
-                    const uint64_t dG = sw128_desc(smem + lay.a_off(sa));
-                    const uint64_t dO = sw128_desc(smem + lay.a_off(sa) + kATile);
-                    const uint64_t dB = sw128_desc(smem + lay.b_off(sb));
+                const uint64_t dG = sw128_desc(smem + lay.a_off(s));
+                const uint64_t dO = dG + (kATile >> 4);
+                const uint64_t dB = sw128_desc(smem + lay.b_off(s));
+                if (elect_one()) {
                     if (complete) {
-                        // No O plane: the G products alternate between two
-                        // accumulators (even K-substeps at column 0, odd ones
-                        // in the O accumulator's columns), summed by the
-                        // epilogue; back-to-back MMAs into one accumulator
-                        // run at about half the rate of two interleaved ones.
 #pragma unroll
                         for (int kk = 0; kk < kBK / 32; ++kk)
-                            umma_i8(tmem + ((kk & 1) ? kOCol : 0u), dG + 2 * kk, dB + 2 * kk, idesc,
-                                    (kt > 0 || kk >= 2) ? 1u : 0u);
+                            umma_i8(acc, dG + 2 * kk, dB + 2 * kk, idesc, (kt | kk) ? 1u : 0u);
                     } else {
 #pragma unroll
                         for (int kk = 0; kk < kBK / 32; ++kk) {
-                            const uint32_t acc = (kt | kk) ? 1u : 0u;
-                            umma_i8(tmem, dG + 2 * kk, dB + 2 * kk, idesc, acc);
-                            umma_i8(tmem + kOCol, dO + 2 * kk, dB + 2 * kk, idesc, acc);
+                            const uint32_t go = (kt | kk) ? 1u : 0u;
+                            umma_i8(tmem, dG + 2 * kk, dB + 2 * kk, idesc, go);
+                            umma_i8(tmem + kOCol, dO + 2 * kk, dB + 2 * kk, idesc, go);
                         }
                     }
-                    umma_commit(&a_empty[sa]);
-                    umma_commit(&b_empty[sb]);
+                    umma_commit(&empty[s]);
                 }
-                umma_commit(acc_full);
+                __syncwarp();
+                if (++s == kStages) { s = 0; ph ^= 1u; }
             }
+            if (ok && elect_one()) umma_commit(&acc_full[b]);
+            __syncwarp();
         }
+        // Drain: every MMA issued here completes before TMEM is released.
+        if (elect_one()) umma_commit(mma_done);
+        __syncwarp();
+        mbar_wait(mma_done, 0u);
     } else {
         // ---------------- decoders (warps 3..) + epilogue (warps 3..6) ----------------
         const int dset = (warp - 3) >> 2;    // decoder set of this warp
@@ -268,6 +292,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         double run2 = 0.0, run4 = 0.0, run2b = 0.0;
         unsigned long long chk_g = 0ULL, chk_o = 0ULL;  // product checksums (a.chk)
         int cur = 0;  // bin offset (within this CTA's bins) that run2/run4 belong to
+        ProbeSlot* const slots =
+            reinterpret_cast<ProbeSlot*>(smem + lay.slot_off()) + ((warp - 3) & 3) * 64;
         // Add the running sums of bin k0 + cur to the outputs, with the
         // reference's guards, and restart them.
         auto flush = [&]() {
@@ -298,111 +324,150 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             run2 = run4 = run2b = 0.0;
         };
-        int it = 0;
+        int it = 0, sp = 0, s = 0;
+        uint32_t php = 0, ph = 0;
         for (int g = 0; g < ngroups; ++g) {
             for (int kt = 0; kt < a.nkt; ++kt, ++it) {
-                if (it % kDecSets != dset) continue;
-                const int sp = it % kPkStages, sa = it % kAStages;
-                // Warp-uniform waits and one arrival per warp (after __syncwarp,
-                // which orders the warp's shared-memory accesses before it):
-                // 4 arrivals per stage instead of 128.
-                if (!__all_sync(0xffffffffu,
-                                mbar_wait(&pk_full[sp], (uint32_t)(it / kPkStages) & 1u))) {
-                    fail(5);
-                    break;
+                if (it % kDecSets == dset) {
+                    // Warp-uniform waits and one arrival per warp (after __syncwarp,
+                    // which orders the warp's shared-memory accesses before it):
+                    // 4 arrivals per stage instead of 128.
+                    if (!warp_wait(&pk_full[sp], php, abort_flag)) {
+                        fail(5);
+                        break;
+                    }
+                    const uint4* pk = reinterpret_cast<const uint4*>(smem + lay.pk_off(sp) + r * 32);
+                    const uint4 p0 = pk[0], p1 = pk[1];
+                    if (it >= kStages && !warp_wait(&empty[s], ph ^ 1u, abort_flag)) {
+                        fail(6);
+                        break;
+                    }
+                    uint8_t* gRow = smem + lay.a_off(s) + (r >> 3) * 1024 + (r & 7) * 128;
+                    if (complete) decode_row_sw128_g(p0, p1, gRow, r);
+                    else decode_row_sw128(p0, p1, gRow, gRow + kATile, r);
+                    // The packed rows go back only now: the decode has used what was
+                    // read, so no read of the slot can still be on its way.
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&pk_empty[sp]);
+                    fence_async_smem();
+                    if (((warp - 3) & 3) == 0 && !warp_wait(&b_full[s], ph, abort_flag)) {
+                        fail(8);
+                        break;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&full[s]);
                 }
-                if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
-                const uint4* pk = reinterpret_cast<const uint4*>(smem + lay.pk_off(sp) + r * 32);
-                const uint4 p0 = pk[0], p1 = pk[1];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&pk_empty[sp]);
-                if (it >= kAStages &&
-                    !__all_sync(0xffffffffu, mbar_wait(&a_empty[sa],
-                                                       ((uint32_t)(it / kAStages) & 1u) ^ 1u))) {
-                    fail(6);
-                    break;
-                }
-                uint8_t* gRow = smem + lay.a_off(sa) + (r >> 3) * 1024 + (r & 7) * 128;
-                if (complete) decode_row_sw128_g(p0, p1, gRow, r);
-                else decode_row_sw128(p0, p1, gRow, gRow + kATile, r);
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[sa]);
+                if (++sp == kPkStages) { sp = 0; php ^= 1u; }
+                if (++s == kStages) { s = 0; ph ^= 1u; }
             }
             if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
             if (dset != 0) continue;
-            // Epilogue of column group g.
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_full, (uint32_t)g & 1u))) {
+            // Epilogue of column group g: this warp's table of the group's 64 probe
+            // slots first, while the last MMAs run.
+            const int ncols = min(256, cols - g * 256);
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int gc = g * 256 + 4 * (lane + 32 * x);   // column within this CTA's bins
+                const int bo = gc / a.ncolp, v = (gc - bo * a.ncolp) >> 2;
+                ProbeSlot ps{0.0, 0LL, -1, v};
+                if (gc < cols && bo < nbk && v < a.V) {
+                    ps.bin = bo;
+                    if (a.colscale) ps.scale = a.colscale[(int64_t)(kb + bo) * a.V + v];
+                    if (complete) {
+                        const int* cs = a.colsum + (int64_t)kb * a.ncolp + gc;
+                        ps.colsum = (((long long)cs[0] * 128 + cs[1]) * 128 + cs[2]) * 128 + cs[3];
+                    }
+                }
+                slots[lane + 32 * x] = ps;
+            }
+            __syncwarp();
+            const int b = complete ? g & 1 : 0, u = complete ? g >> 1 : g;
+            if (!warp_wait(&acc_full[b], (uint32_t)u & 1u, abort_flag)) {
                 fail(7);
                 break;
             }
             tc_fence_after();
-            const int ncols = min(256, cols - g * 256);
-            const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16);
+            const uint32_t tbase = tmem + (uint32_t)b * kOCol + ((uint32_t)(q * 32) << 16);
             for (int c0 = 0; c0 < ncols; c0 += 32) {
                 int rg[32], ro[32];
+                __syncwarp();
                 tmem_ld32(tbase + (uint32_t)c0, rg);
-                tmem_ld32(tbase + kOCol + (uint32_t)c0, ro);
-                tmem_wait_ld();
-                if (complete) {
-                    // the G products' second accumulator, then every call
-                    // observed: O^T y = the digit columns' sums (columns past
-                    // this CTA's bins belong to no output)
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) rg[q] += ro[q];
-                    const int live = min(ncols, nbk * a.ncolp - g * 256) - c0;
-                    const int* cs = a.colsum + (int64_t)kb * a.ncolp + g * 256 + c0;
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) ro[q] = q < live ? cs[q] : 0;
+                if (!complete) {
+                    tmem_ld32(tbase + kOCol + (uint32_t)c0, ro);
+                    tmem_wait_ld(ro);
                 }
-                // Checksum weights of the chunk's 8 probes: lane p hashes
-                // probe p's, the loop below broadcasts them.
-                unsigned long long hl = 0ULL;
-                if (a.chk) {
-                    const int gcl = g * 256 + c0 + 4 * (lane & 7);
-                    const int bol = gcl / a.ncolp;
-                    hl = check_weight(k0 + bol, a.chk_v0 + ((gcl - bol * a.ncolp) >> 2));
-                }
+                tmem_wait_ld(rg);
+                // All eight probes' products and scaled values before any sum or
+                // output: a bin's flush in between would chain the probes' table
+                // reads and FP64 work one after another (38,000 cycles per group).
+                const ProbeSlot* const sl = slots + (c0 >> 2);
+                long long TG[8], TO[8];
+                double wv[8];
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
-                    const unsigned long long h = a.chk ? __shfl_sync(0xffffffffu, hl, p) : 0ULL;
-                    const int gc = g * 256 + c0 + 4 * p;   // column within this CTA's bins
-                    const int bo = gc / a.ncolp;            // bin offset (warp-uniform)
-                    const int v = (gc - bo * a.ncolp) >> 2;
-                    if (bo >= nbk || v >= a.V) continue;
-                    if (bo != cur) {
-                        flush();
-                        cur = bo;
-                    }
-                    const long long TG =
-                        (((long long)rg[4 * p] * 128 + rg[4 * p + 1]) * 128 + rg[4 * p + 2]) * 128 +
-                        rg[4 * p + 3];
-                    const long long TO =
-                        (((long long)ro[4 * p] * 128 + ro[4 * p + 1]) * 128 + ro[4 * p + 2]) * 128 +
-                        ro[4 * p + 3];
-                    if (a.chk) {
-                        chk_g += h * (unsigned long long)TG;
-                        chk_o += h * (unsigned long long)TO;
-                    }
-                    if (a.raw_g) {
-                        if (j < jend) {
-                            const int64_t ro = ((j - a.out_row0) * a.K + k0 + bo) * a.V + v;
-                            a.raw_g[ro] = TG;
-                            a.raw_o[ro] = TO;
+                    TG[p] = (((long long)rg[4 * p] * 128 + rg[4 * p + 1]) * 128 + rg[4 * p + 2]) * 128 +
+                            rg[4 * p + 3];
+                    // without a missing call, O^T y = the digit columns' sums
+                    TO[p] = complete ? sl[p].colsum
+                                     : (((long long)ro[4 * p] * 128 + ro[4 * p + 1]) * 128 +
+                                        ro[4 * p + 2]) * 128 + ro[4 * p + 3];
+                    wv[p] = sd * sl[p].scale * ((double)TG[p] - mu * (double)TO[p]);
+                }
+                if (a.raw_g || a.chk) {
+                    // Checksum weights of the chunk's 8 probes: lane p hashes
+                    // probe p's, the loop below broadcasts them.
+                    unsigned long long hl = 0ULL;
+                    if (a.chk)
+                        hl = check_weight(k0 + max(sl[lane & 7].bin, 0), a.chk_v0 + sl[lane & 7].v);
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        const unsigned long long h = a.chk ? __shfl_sync(0xffffffffu, hl, p) : 0ULL;
+                        if (sl[p].bin < 0) continue;
+                        chk_g += h * (unsigned long long)TG[p];
+                        chk_o += h * (unsigned long long)TO[p];
+                        if (a.raw_g && j < jend) {
+                            const int64_t o =
+                                ((j - a.out_row0) * a.K + k0 + sl[p].bin) * a.V + sl[p].v;
+                            a.raw_g[o] = TG[p];
+                            a.raw_o[o] = TO[p];
                         }
-                        continue;
                     }
-                    const double wv = sd * a.colscale[(int64_t)(kb + bo) * a.V + v] *
-                                      ((double)TG - mu * (double)TO);
-                    const double w2 = wv * wv;
-                    if (a.accum2 && v >= a.split_v) run2b += w2;
-                    else run2 += w2;
-                    run4 += w2 * w2;
+                    if (a.raw_g) continue;
+                }
+                // The sums, in probe order.  One bin without the half split is the
+                // common chunk; a bin's end inside the chunk flushes.
+                const int b0 = sl[0].bin;
+                if (b0 >= 0 && b0 == sl[7].bin && !a.accum2) {
+                    if (b0 != cur) {
+                        flush();
+                        cur = b0;
+                    }
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        const double w2 = wv[p] * wv[p];
+                        run2 += w2;
+                        run4 += w2 * w2;
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        const int bo = sl[p].bin;   // (warp-uniform)
+                        if (bo < 0) continue;
+                        if (bo != cur) {
+                            flush();
+                            cur = bo;
+                        }
+                        const double w2 = wv[p] * wv[p];
+                        if (a.accum2 && sl[p].v >= a.split_v) run2b += w2;
+                        else run2 += w2;
+                        run4 += w2 * w2;
+                    }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty);
+            if (lane == 0) mbar_arrive(&acc_empty[b]);
         }
         if (dset == 0) {
             flush();

@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     for (int c0 = 32 * h, cc = 0; c0 < ncols; c0 += 128, cc += 8) {
                         int rr[32];
                         tmem_ld32(tbase + (uint32_t)c0, rr);
-                        tmem_wait_ld();
+                        tmem_wait_ld(rr);
                         const int v0 = g * 64 + (c0 >> 2);          // first probe of the chunk (even)
                         const int nv = a.V - v0;                    // probes left (warp-uniform)
                         // All roundings before the first store: a store in between
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                 for (int c0c = 16 * h; c0c < ncols; c0c += 64) {
                     int rr[16];
                     tmem_ld16(tbase + (uint32_t)c0c, rr);
-                    tmem_wait_ld();
+                    tmem_wait_ld(rr);
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
                         const int vl = c0c / 4 + p;  // probe within the group (warp-uniform)
