@@ -1740,7 +1740,6 @@ struct GwPlan {
         Csr csr;
         DevBuf rowind, sc, binoff, wqoff, z, wq, wcs;
         int64_t lmax = 0;     // tcgen05 phase 1: padded member-list length
-        CUtensorMap tmW;      // tcgen05 phase 1: weight digits
     };
     std::vector<std::unique_ptr<Tile>> tiles;
     DevBuf y, yq, ycs, accum, mc, lscale, guards, status;
@@ -1844,7 +1843,7 @@ std::unique_ptr<GwPlan> plan_create(Context& c, std::shared_ptr<Prepared> P, con
         t->V = V;
         t->Vp = (int)round_up(V, kColTile);
         const bool tc = (p2_impl() == 1 && pl->S == 4);
-        const int64_t pad = tc ? 128 : kSnpStep;
+        const int64_t pad = tc ? umma::kP1Step : kSnpStep;
         const uint8_t* cst = P->constant.data();
         t->csr = as_float
             ? build_csr<float>(annot_f.data(), inv_f.data(), M, K, 0, t->Vp, pl->S, pad, cst)
@@ -1891,14 +1890,9 @@ std::unique_ptr<GwPlan> plan_create(Context& c, std::shared_ptr<Prepared> P, con
         if (tc) {
             for (int64_t kk = 0; kk < K; ++kk)
                 t->lmax = std::max(t->lmax, cs.bin_off[(size_t)kk + 1] - cs.bin_off[(size_t)kk]);
-            t->lmax = std::max<int64_t>(t->lmax, 128);
-            const int nc = umma::ncolp_for(V);
-            const size_t bytes = (size_t)(K * 2 * nc) * (size_t)t->lmax;
-            int8_t* wq = t->wq.as<int8_t>(bytes);
-            ck(cudaMemsetAsync(wq, 0, bytes, c.st), "memset weights");
+            t->wq.as<int8_t>(std::max<size_t>(
+                umma::w_digit_bytes(cs.bin_off[(size_t)K], umma::ncolp_for(V)), 16));
             t->wcs.as<double>((size_t)(K * V));
-            t->tmW = make_map_2d(wq, (uint64_t)t->lmax, (uint64_t)(K * 2 * nc), (uint64_t)t->lmax,
-                                 128, (uint32_t)std::min(256, nc), CU_TENSOR_MAP_SWIZZLE_128B);
         } else {
             t->wq.as<int8_t>((size_t)std::max<int64_t>(cs.wq_bytes, 16));
             t->wcs.as<double>((size_t)(K * t->Vp));
@@ -2000,7 +1994,7 @@ void plan_enqueue_phase1(Context& c, GwPlan& pl, size_t ti, double* y, cudaEvent
         pa.V = t.V;
         pa.ncolp = nc;
         pa.ngroups = (nc + 255) / 256;
-        pa.box_rows = std::min(256, nc);
+        pa.wq = uw.wq;
         pa.nbp = P.g.nbp;
         pa.N_pad = P.g.N_pad;
         pa.bin_off = w.bin_off;
@@ -2011,7 +2005,7 @@ void plan_enqueue_phase1(Context& c, GwPlan& pl, size_t ti, double* y, cudaEvent
         pa.status = static_cast<unsigned*>(pl.status.p);
         pa.m_pad = P.g.M_pad;
         pa.lmax = t.lmax;
-        umma::launch_p1_umma(t.tmW, pa, P.g.N_pad, c.st);
+        umma::launch_p1_umma(pa, P.g.N_pad, c.st);
     } else {
         launch_p1_weights(w, static_cast<double*>(P.d_mean.p), static_cast<double*>(P.d_sdinv.p),
                           static_cast<double*>(t.z.p), M, 0, c.st);
@@ -2436,8 +2430,10 @@ std::unique_ptr<WinPlan> win_plan_create(Context& c, std::shared_ptr<Prepared> P
         const int64_t a0 = ws[w], L = ws[w + 1] - ws[w];
         const uint8_t* cst = P->constant.data();
         parts[(size_t)w] = as_float
-            ? build_csr<float>(annot_f.data() + a0 * K, inv_f.data() + a0, L, K, a0, 16, 4, 128, cst)
-            : build_csr<double>(annot + a0 * K, pl->inv.data() + a0, L, K, a0, 16, 4, 128, cst);
+            ? build_csr<float>(annot_f.data() + a0 * K, inv_f.data() + a0, L, K, a0, 16, 4,
+                               umma::kP1Step, cst)
+            : build_csr<double>(annot + a0 * K, pl->inv.data() + a0, L, K, a0, 16, 4,
+                                umma::kP1Step, cst);
     });
     int64_t max_ksup = 0, max_wq = 0;
     for (int64_t w0 = 0; w0 < W; w0 += wb) {
@@ -2466,7 +2462,6 @@ std::unique_ptr<WinPlan> win_plan_create(Context& c, std::shared_ptr<Prepared> P
             }
         }
         cs.bin_off[(size_t)b.ksup] = off;
-        b.lmax = std::max<int64_t>(b.lmax, 128);
         const size_t nm = std::max<size_t>(ri.size(), 1);
         h2d(b.rowind.as<int32_t>(nm), ri.data(), ri.size(), c.st);
         h2d(b.sc.as<double>(nm), scv.data(), scv.size(), c.st);
@@ -2485,7 +2480,7 @@ std::unique_ptr<WinPlan> win_plan_create(Context& c, std::shared_ptr<Prepared> P
         build_win_work(c, *pl, b);
         ck(cudaStreamSynchronize(c.st), "window batch upload");
         max_ksup = std::max(max_ksup, b.ksup);
-        max_wq = std::max(max_wq, b.ksup * 2 * ncmax * b.lmax);
+        max_wq = std::max(max_wq, (int64_t)umma::w_digit_bytes(off, ncmax));
         b.csr.nnz = cs.nnz;
         pl->batches.push_back(std::move(b));
     }
@@ -2606,21 +2601,16 @@ void win_enqueue(Context& c, WinPlan& pl) {
             uw.colscale = static_cast<double*>(pl.wcs.p);
             uw.ycolscale = static_cast<double*>(pl.ycs.p);
             uw.yshift = static_cast<int*>(pl.yshift.p);
-            const size_t wbytes = (size_t)(b.ksup * 2 * nc) * (size_t)b.lmax;
-            ck(cudaMemsetAsync(pl.wq->p, 0, wbytes, c.st), "memset weights");
             umma::launch_p1_weights4(uw, static_cast<double*>(P.d_mean.p),
                                      static_cast<double*>(P.d_sdinv.p),
                                      static_cast<double*>(pl.z[ti].p), M, c.st);
             ck(cudaEventRecordWithFlags(pl.ev[(size_t)e++], c.st, cudaEventRecordExternal), "event");
-            const CUtensorMap tmW =
-                make_map_2d(pl.wq->p, (uint64_t)b.lmax, (uint64_t)(b.ksup * 2 * nc), (uint64_t)b.lmax,
-                            128, (uint32_t)std::min(256, nc), CU_TENSOR_MAP_SWIZZLE_128B);
             umma::P1UArgs pa;
             pa.K = (int)b.ksup;
             pa.V = V;
             pa.ncolp = nc;
             pa.ngroups = (nc + 255) / 256;
-            pa.box_rows = std::min(256, nc);
+            pa.wq = uw.wq;
             pa.nbp = P.g.nbp;
             pa.N_pad = Np;
             pa.bin_off = uw.bin_off;
@@ -2639,7 +2629,7 @@ void win_enqueue(Context& c, WinPlan& pl) {
             pa.ycolscale = static_cast<double*>(pl.ycs.p);
             pa.yshift = static_cast<int*>(pl.yshift.p);
             pa.m_pad = P.g.M_pad;
-            umma::launch_p1_umma(tmW, pa, Np, c.st);
+            umma::launch_p1_umma(pa, Np, c.st);
             ck(cudaEventRecordWithFlags(pl.ev[(size_t)e++], c.st, cudaEventRecordExternal), "event");
             // (sketch digits were written by phase 1's epilogue; their column
             // sums stand in for the O plane of tiles without missing calls)
@@ -3295,7 +3285,7 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         std::vector<int64_t> off((size_t)G + 1, 0);
         std::vector<int32_t> ri;
         std::vector<double> scv;
-        int64_t lmax = 128;
+        int64_t lmax = umma::kP1Step;
         for (int64_t e = 0; e < T; ++e)
             for (int h = 0; h < 2; ++h)
                 for (int64_t k = 0; k < K; ++k) {
@@ -3310,7 +3300,7 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
                         scv.push_back(sa * s[j]);
                     }
                     const int64_t n = (int64_t)ri.size() - off[(size_t)gi];
-                    const int64_t np = round_up(n, 128);
+                    const int64_t np = round_up(n, umma::kP1Step);
                     for (int64_t q = n; q < np; ++q) {
                         ri.push_back(0);
                         scv.push_back(0.0);
@@ -3322,9 +3312,7 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         h2d(g.rowind.as<int32_t>(nm), ri.data(), ri.size(), c.st);
         h2d(g.sc.as<double>(nm), scv.data(), scv.size(), c.st);
         h2d(g.binoff.as<int64_t>(off.size()), off.data(), off.size(), c.st);
-        const size_t wbytes = (size_t)(G * 2 * nc) * (size_t)lmax;
-        int8_t* wq = g.wq.as<int8_t>(wbytes);
-        ck(cudaMemsetAsync(wq, 0, wbytes, c.st), "memset weights");
+        int8_t* wq = g.wq.as<int8_t>(std::max<size_t>(umma::w_digit_bytes((int64_t)ri.size(), nc), 16));
         umma::P1UWeights uw;
         uw.K = (int)G;
         uw.V = (int)B;
@@ -3338,15 +3326,12 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         const double* mean = static_cast<const double*>(P.d_mean.p) + j0 + a;
         const double* sdinv = static_cast<const double*>(P.d_sdinv.p) + j0 + a;
         umma::launch_p1_weights4(uw, mean, sdinv, dz + a, L, c.st);
-        const CUtensorMap tmW = make_map_2d(wq, (uint64_t)lmax, (uint64_t)(G * 2 * nc), (uint64_t)lmax,
-                                            128, (uint32_t)std::min(256, nc),
-                                            CU_TENSOR_MAP_SWIZZLE_128B);
         umma::P1UArgs pa;
         pa.K = (int)G;
         pa.V = (int)B;
         pa.ncolp = nc;
         pa.ngroups = (nc + 255) / 256;
-        pa.box_rows = std::min(256, nc);
+        pa.wq = wq;
         pa.nbp = P.g.nbp;
         pa.N_pad = Np;
         pa.bin_off = uw.bin_off;
@@ -3365,7 +3350,7 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         }
         pa.status = g.status.as<unsigned>(1);
         ck(cudaMemsetAsync(pa.status, 0, 4, c.st), "memset");
-        umma::launch_p1_umma(tmW, pa, Np, c.st);
+        umma::launch_p1_umma(pa, Np, c.st);
         launch_gxe_source_finalize(Y, N, Np, C, (int)(K * B), static_cast<double*>(g.env.p), N,
                                    env_start, dtarget, N, c.st);
         unsigned stv = 0;

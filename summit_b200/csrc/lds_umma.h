@@ -106,12 +106,28 @@ inline int p2_bins_per_cta_grouped(int ncolp, int K) {
     return best;
 }
 
+// Member SNPs per phase-1 K-step: member lists are padded to a multiple of it.
+constexpr int kP1Step = 64;
+
+// Phase-1 weight digits, column col of part 0 (W1) or 1 (-W2) for member r of
+// K-step `step` (counted over all super-bins' lists): a step's columns are
+// contiguous 128-byte rows, the step's members of W1 and then of -W2,
+// pre-swizzled as the SWIZZLE_128B K-major UMMA atom expects (16-byte chunk XOR
+// row & 7).
+__host__ __device__ inline int64_t w_digit_offset(int64_t step, int part, int col, int r,
+                                                  int ncolp) {
+    return (step * ncolp + col) * 2 * kP1Step + (((part * 4 + (r >> 4)) ^ (col & 7)) << 4) + (r & 15);
+}
+// Bytes of the weight digits of `members` list entries (padding included).
+inline size_t w_digit_bytes(int64_t members, int ncolp) { return (size_t)members * 2 * ncolp; }
+
 // Phase-1 tcgen05 kernel arguments.  Member lists of bin k occupy
-// rowind[bin_off[k] .. bin_off[k+1]) (multiples of 128, padding rows carry
-// zero weights); weight digits Wq[((k*2+part)*ncolp + 4v+t)*lmax + r].
+// rowind[bin_off[k] .. bin_off[k+1]) (multiples of kP1Step, padding rows carry
+// zero weights).
 struct P1UArgs {
-    int K = 0, V = 0, ncolp = 0, ngroups = 1, box_rows = 0;
+    int K = 0, V = 0, ncolp = 0, ngroups = 1;
     int64_t nbp = 0, N_pad = 0;
+    const int8_t* wq = nullptr;         // weight digits (w_digit_offset)
     const int64_t* bin_off = nullptr;
     const int32_t* rowind = nullptr;
     const uint8_t* codes = nullptr;
@@ -136,12 +152,12 @@ struct P1UArgs {
 
 // Rows of a weight-digit tile in shared memory.
 __host__ __device__ inline int p1_tile_rows(const P1UArgs& a) {
-    return a.share > 1 ? a.share * a.ncolp : a.box_rows;
+    return a.share > 1 ? a.share * a.ncolp : (a.ncolp < 256 ? a.ncolp : 256);
 }
 
 struct P1UWeights {
     int K = 0, V = 0, ncolp = 0;
-    int64_t lmax = 0;
+    int64_t lmax = 0;                   // longest padded list
     const int32_t* rowind = nullptr;
     const double* sc = nullptr;
     const int64_t* bin_off = nullptr;
@@ -154,7 +170,7 @@ struct P1UWeights {
 void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* sdinv,
                         const double* Z, int64_t z_ld, cudaStream_t st);
 size_t p1_umma_smem_bytes(int tile_rows);
-void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cudaStream_t st);
+void launch_p1_umma(const P1UArgs& a, int64_t N_pad, cudaStream_t st);
 
 // Columns per bin (4 digits per probe, padded to a multiple of 16).
 inline int ncolp_for(int V) { return ((4 * V + 15) / 16) * 16; }

@@ -1,27 +1,34 @@
 // Phase 1 on tcgen05 tensor cores: Y[:, (k, v)] = sum_{j in bin k} x_j w_{j,(k,v)}.
 //
 // UMMA shape per CTA: M = 128 samples, N = the bin's digit columns (4 per
-// probe, <= 256 per pass), K = 128 member SNPs per stage.  The A operand is
+// probe, <= 256 per pass), K = 64 member SNPs per stage.  The A operand is
 // the decoded genotype tile in MN-major SWIZZLE_128B layout: a packed SNP row
 // already lists samples contiguously, so decoder thread t expands member SNP t
 // of the stage into row t of the tile with no transpose.  G and O tiles are
-// multiplied by the digits of W1 = s_j sc z and of -W2 = -mu_j W1 (both via
-// TMA, SWIZZLE_128B, K-major) into ONE accumulator, so TMEM holds
-// G.W1 - O.W2 = sum_j (g - mu_j o) s_j sc z directly.
+// multiplied by the digits of W1 = s_j sc z and of -W2 = -mu_j W1 (side by side
+// in 128-byte rows, SWIZZLE_128B, K-major, laid out contiguous by the weight
+// kernel, w_digit_offset, so that one bulk copy brings a K-step's tile) into ONE
+// accumulator, so TMEM holds G.W1 - O.W2 = sum_j (g - mu_j o) s_j sc z directly.
 //
 // Roles (832 threads): warp 0 TMA producer for the digit tiles; warp 1 TMEM
-// allocation and the single MMA-issuing thread; warps 2-9, two decoder sets of
-// four (set d takes the K-steps of its parity), gather the member SNPs' packed
+// allocation and the single MMA-issuing thread; warps 2-9, four decoder sets of
+// two (set d takes the K-steps it with it % 4 == d), gather the member SNPs' packed
 // bytes from global memory (one row each, kept several steps ahead by
-// cp.async) and decode them into the operand tiles; warps 10-25 (four per TMEM
-// lane quadrant) read the accumulator out and split it into digits.  Two TMEM
-// accumulators let the MMAs of the next job (super-bin, column group) run while
-// the epilogue of the previous one drains, which matters for windowed
-// estimates, whose super-bins are a few K-steps long.
+// cp.async) and decode them into the operand tiles; warps 10-25, eight per TMEM
+// accumulator, read it out and split it into digits.  Two TMEM accumulators let
+// the MMAs of the next job (super-bin, column group) run while the epilogue of
+// the previous one drains, which matters for windowed estimates, whose super-bins
+// are a few K-steps long.
 //
-// What bounds it: with many K-steps per super-bin the decode (one set of four
-// warps held a K-step at 2,007 cycles against 832 of MMA at N = 208); with few,
-// the digit epilogue's instructions per (sample, probe).
+// What bounds it: with many K-steps per super-bin the weight tiles' L2 reads
+// (26.6 KB per 64 members and sample tile at N = 208, about 10 TB/s over the
+// chip); with few, the digit epilogue and the latency from a stage's release to
+// its next tiles.  Stages of 64 members and not 128 give four and not two of
+// them in 227 KB, and short lists less padding; the issuing warp's loop is
+// warp-uniform with one wait per K-step (a single diverged thread with two waits
+// took 640 cycles per K-step beside 416 of MMA).  Windowed, N = 50,000,
+// M = 60,000, K = 24, B = 50: 8.7 -> 8.2 ms; N = 10,007, K = 6, B = 10: 137 ->
+// 115 us; N = 200,003, K = 1, B = 50: 1.19 -> 1.07 ms.
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -35,54 +42,57 @@ namespace lds {
 namespace umma {
 
 namespace p1 {
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 8;
 constexpr int kBM = 128;          // samples per CTA
-constexpr int kBK = 128;          // member SNPs per stage
-constexpr int kATile = 128 * 128; // 16 KB
-constexpr int kDecSets = 2;
+constexpr int kBK = kP1Step;      // member SNPs per stage (64)
+constexpr int kATile = kBM * kBK; // 8 KB
+constexpr int kDecSets = 4;
+constexpr int kSetWarps = kBK / 32;      // a decoder thread per member row
 constexpr int kDecWarp0 = 2;
-constexpr int kEpiWarp0 = kDecWarp0 + 4 * kDecSets;
-constexpr int kEpiWarps = 16;            // four per TMEM lane quadrant
+constexpr int kEpiWarp0 = kDecWarp0 + kSetWarps * kDecSets;
+constexpr int kEpiWarps = 8;             // per accumulator: two per TMEM lane quadrant
 constexpr int kEpiThreads = 32 * kEpiWarps;
-constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
+constexpr int kThreads = 32 * (kEpiWarp0 + 2 * kEpiWarps);
 constexpr int kAccCols = 256;            // one accumulator: <= 256 digit columns
 constexpr uint32_t kTmemCols = 512;      // two accumulators (MMA of job j+1 || epilogue of j)
-constexpr int kRing = 6;                 // K-steps whose packed rows are in flight
-constexpr int kRingSlot = 128 * 32;      // 128 member rows x 32 bytes
+constexpr int kDepth = 3;                // gathered K-steps in flight per decoder set
+constexpr int kRing = kDepth * kDecSets; // ring slots
+constexpr int kRingSlot = kBK * 32;      // a K-step's member rows x 32 bytes
 constexpr int kMaxSb = 256;              // super-bins per CTA (their offsets in shared memory)
+constexpr int kShiftBytes = 2 * kEpiWarps * 32 * 16;  // digit shifts of 32 probes per epilogue warp
 constexpr int kSmemLimit = 227 * 1024;
 // Longest list whose |128 t2 + t3| stays below 2^31: the low digits' products
 // are at most 3 * 64 per member.
 constexpr int kMaxNarrowSteps = 86000 / kBK;
 
-// Shared memory: the stages (G and O tiles, then the two weight-digit tiles of
-// box_rows columns), the gather ring, the barriers, the super-bin table, and
+// Shared memory: the stages (G and O tiles, then the weight-digit tile of
+// tile_rows columns), the gather ring, the barriers, the super-bin table, and
 // each epilogue warp's digit-shift table.
 struct Layout {
-    uint32_t w_tile, stage;
+    uint32_t stage;
     int stages;
-    __host__ __device__ explicit Layout(int box_rows)
-        : w_tile((uint32_t)((box_rows * kBK + 1023) / 1024 * 1024)),
-          stage(2 * kATile + 2 * w_tile),
+    __host__ __device__ explicit Layout(int tile_rows)
+        : stage(2 * kATile + (uint32_t)((tile_rows * 2 * kBK + 1023) / 1024 * 1024)),
           stages(0) {
         const int fit = (int)((kSmemLimit - 1024 - tail()) / stage);
         stages = fit < kMaxStages ? fit : kMaxStages;
     }
     __host__ __device__ static constexpr uint32_t tail() {
-        return kRing * kRingSlot + 256 + (kMaxSb + 4) * 4 + kEpiWarps * 16 * 16;
+        return kRing * kRingSlot + 256 + (kMaxSb + 4) * 4 + kShiftBytes;
     }
     __host__ __device__ uint32_t ring_off() const { return (uint32_t)stages * stage; }
     __host__ __device__ uint32_t bar_off() const { return ring_off() + kRing * kRingSlot; }
     __host__ __device__ uint32_t shift_off() const { return bar_off() + 256; }
-    __host__ __device__ uint32_t table_off() const { return shift_off() + kEpiWarps * 16 * 16; }
+    __host__ __device__ uint32_t table_off() const { return shift_off() + kShiftBytes; }
     __host__ __device__ uint32_t bytes() const { return ring_off() + tail(); }
 };
-static_assert(2 * (2 * kATile + 2 * 256 * kBK) + Layout::tail() + 1024 <= kSmemLimit,
-              "two stages of 256 digit columns fit");
+static_assert(4 * (2 * kATile + 2 * 256 * kBK) + Layout::tail() + 1024 <= kSmemLimit,
+              "four stages of 256 digit columns fit");
+static_assert((2 * kMaxStages + 5) * 8 + 8 <= 256, "the barriers fit");
 }  // namespace p1
 
 __global__ void __launch_bounds__(p1::kThreads, 1)
-    p1_umma_kernel(const __grid_constant__ CUtensorMap tmW, P1UArgs a) {
+    p1_umma_kernel(P1UArgs a) {
     using namespace p1;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
@@ -90,10 +100,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     const int nst = lay.stages;
     uint8_t* ring = smem + lay.ring_off();
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bar_off());
-    uint64_t* full_w = bars;                    // [nst] weight tiles landed (TMA)
-    uint64_t* full_dec = bars + kMaxStages;     // [nst] genotype tiles decoded
-    uint64_t* empty = bars + 2 * kMaxStages;    // [nst] stage consumed by the MMAs
-    uint64_t* acc_full = bars + 3 * kMaxStages; // [2] accumulator b holds a finished job
+    uint64_t* full = bars;                      // [nst] genotype tiles decoded, weight tile landed
+    uint64_t* empty = bars + kMaxStages;        // [nst] stage consumed by the MMAs
+    uint64_t* acc_full = bars + 2 * kMaxStages; // [2] accumulator b holds a finished job
     uint64_t* acc_empty = acc_full + 2;         // [2] accumulator b read out
     uint64_t* mma_done = acc_empty + 2;         // drain of the issuer's MMAs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
@@ -101,7 +110,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     int4* shift_tab = reinterpret_cast<int4*>(smem + lay.shift_off());
     int* ktab = reinterpret_cast<int*>(smem + lay.table_off());
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int64_t i0 = (int64_t)blockIdx.x * kBM;
     // This CTA's super-bins: kb0 .. kb0 + nsb; a job is one (super-bin, column
     // group), or with share > 1 that many super-bins with one member list, their
@@ -113,8 +122,8 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     for (int q = tid; q <= nsb; q += kThreads) ktab[q] = (int)(a.bin_off[kb0 + q] / kBK);
     if (tid == 0) {
         for (int s = 0; s < nst; ++s) {
-            mbar_init(&full_w[s], 1);
-            mbar_init(&full_dec[s], 4);            // one arrival per decoder warp of the step's set
+            // the step's decoder warps, and the weight producer with its copies' bytes
+            mbar_init(&full[s], kSetWarps + 1);
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -161,16 +170,15 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                 const int nkt = steps_of(q, k0), nbin = min(a.share, nsb - q);
                 for (int g = 0; g < a.ngroups && !*abort_flag; ++g) {
                     for (int kt = 0; kt < nkt; ++kt, ++it) {
-                        if (it >= nst && !mbar_wait(&empty[s], ph ^ 1u)) { fail(11); break; }
-                        if (*abort_flag) break;
+                        if (it >= nst && !mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { fail(11); break; }
                         uint8_t* w = smem + s * lay.stage + 2 * kATile;
-                        mbar_expect_tx(&full_w[s], (uint32_t)(2 * nbin * a.box_rows * kBK));
-                        for (int u = 0; u < nbin; ++u, w += a.ncolp * kBK) {
-                            const int y0 = (kb0 + q + u) * 2 * a.ncolp + g * 256;
-                            tma_load_2d(w, &tmW, (k0 + kt) * kBK, y0, &full_w[s]);
-                            tma_load_2d(w + lay.w_tile, &tmW, (k0 + kt) * kBK, y0 + a.ncolp,
-                                        &full_w[s]);
-                        }
+                        // the group's columns, for each bin of the job
+                        const uint32_t bytes = (uint32_t)min(256, a.ncolp - g * 256) * 2 * kBK;
+                        mbar_expect_tx(&full[s], (uint32_t)nbin * bytes);
+                        for (int u = 0; u < nbin; ++u, w += a.ncolp * 2 * kBK)
+                            bulk_load(w, a.wq + ((int64_t)(ktab[q + u] + k0 + kt) * a.ncolp + g * 256) *
+                                                    2 * kBK,
+                                      bytes, &full[s]);
                         if (++s == nst) { s = 0; ph ^= 1u; }
                     }
                 }
@@ -178,37 +186,44 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             // Drain: no tile copy may still be landing when the CTA exits
             // (only reachable with copies outstanding after an abort).
             for (int j = max(0, it - nst); j < it; ++j)
-                mbar_wait(&full_w[j % nst], (uint32_t)(j / nst) & 1u);
+                mbar_wait(&full[j % nst], (uint32_t)(j / nst) & 1u);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int s = 0, au = 0;  // stage, jobs (accumulator uses)
-            uint32_t ph = 0;
-            for (int q = 0; q < nsb && !*abort_flag; q += a.share) {
-                int k0;
-                const int nkt = steps_of(q, k0);
-                const int width = min(a.share, nsb - q) * a.ncolp;   // the job's digit columns
-                if (nkt == 0) continue;
-                for (int g = 0; g < a.ngroups && !*abort_flag; ++g, ++au) {
-                    const int b = au & 1, u = au >> 1;
-                    const int ncols = min(kAccCols, width - g * 256);
-                    const uint32_t idesc = idesc_i8_amn(kBM, ncols);
-                    const uint32_t acc = tmem + (uint32_t)(b * kAccCols);
-                    if (u > 0 && !mbar_wait(&acc_empty[b], (uint32_t)(u - 1) & 1u)) { fail(12); break; }
+        // The whole warp walks the loop (so that addresses, phases and
+        // descriptors stay in uniform registers); one elected thread issues.
+        int s = 0, au = 0;  // stage, jobs (accumulator uses)
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int q = 0; q < nsb && ok; q += a.share) {
+            int k0;
+            const int nkt = steps_of(q, k0);
+            const int width = min(a.share, nsb - q) * a.ncolp;   // the job's digit columns
+            if (nkt == 0) continue;
+            for (int g = 0; g < a.ngroups && ok; ++g, ++au) {
+                const int b = au & 1, u = au >> 1;
+                const int ncols = min(kAccCols, width - g * 256);
+                const uint32_t idesc = idesc_i8_amn(kBM, ncols);
+                const uint32_t acc = tmem + (uint32_t)(b * kAccCols);
+                if (u > 0 && !warp_wait(&acc_empty[b], (uint32_t)(u - 1) & 1u, abort_flag)) {
+                    fail(12);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                for (int kt = 0; kt < nkt; ++kt) {
+                    if (!warp_wait(&full[s], ph, abort_flag)) {
+                        fail(13);
+                        ok = false;
+                        break;
+                    }
                     tc_fence_after();
-                    for (int kt = 0; kt < nkt; ++kt) {
-                        if (!mbar_wait(&full_dec[s], ph) || !mbar_wait(&full_w[s], ph)) {
-                            fail(13);
-                            break;
-                        }
-                        if (*abort_flag) break;
-                        tc_fence_after();
-                        uint8_t* st = smem + s * lay.stage;
-                        const uint64_t dG = sw128_desc_mn(st);
-                        const uint64_t dO = sw128_desc_mn(st + kATile);
-                        const uint64_t dW1 = sw128_desc(st + 2 * kATile);
-                        const uint64_t dW2 = sw128_desc(st + 2 * kATile + lay.w_tile);
+                    uint8_t* st = smem + s * lay.stage;
+                    const uint64_t dG = sw128_desc_mn(st);
+                    const uint64_t dO = sw128_desc_mn(st + kATile);
+                    const uint64_t dW1 = sw128_desc(st + 2 * kATile);
+                    const uint64_t dW2 = dW1 + kBK / 16;
+                    if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < kBK / 32; ++kk) {
                             // A advances 32 K-rows = 4 swizzle atoms (4 KB); B advances 32 bytes.
@@ -216,21 +231,22 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                             umma_i8(acc, dO + 256 * kk, dW2 + 2 * kk, idesc, 1u);
                         }
                         umma_commit(&empty[s]);
-                        if (++s == nst) { s = 0; ph ^= 1u; }
                     }
-                    umma_commit(&acc_full[b]);
+                    __syncwarp();
+                    if (++s == nst) { s = 0; ph ^= 1u; }
                 }
+                if (ok && elect_one()) umma_commit(&acc_full[b]);
+                __syncwarp();
             }
-            // Drain: every MMA issued here completes before TMEM is released.
-            umma_commit(mma_done);
-            mbar_wait(mma_done, 0u);
         }
+        // Drain: every MMA issued here completes before TMEM is released.
+        if (elect_one()) umma_commit(mma_done);
+        __syncwarp();
+        mbar_wait(mma_done, 0u);
     } else if (warp < kEpiWarp0) {
-        // ---------------- gather + decode (two sets of four warps) ----------------
-        // Set d decodes the K-steps it with it % 2 == d, so two operand tiles
-        // are in the making while the MMAs read a third.
-        const int dset = (warp - kDecWarp0) >> 2;
-        const int t = (tid - 32 * kDecWarp0) & 127;
+        // ---------------- gather + decode (four sets of two warps) ----------------
+        const int dset = (warp - kDecWarp0) / kSetWarps;
+        const int t = (tid - 32 * kDecWarp0) % kBK;
         const uint8_t* codes = a.codes + i0 / 4;
         // Gather prefetcher: walks the same (super-bin, group, K-step) sequence
         // ahead of the decode, copying this thread's member row of the set's
@@ -258,37 +274,36 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             } while (pn == 0);
             prow = a.rowind + ((int64_t)(ktab[pq] + k0) * kBK + t);
         };
-        auto cursor_row = [&]() -> int64_t {  // member row of the set's next step, or -1
+        auto cursor_row = [&]() -> int32_t {  // member row of the set's next step, or -1
             advance();
             if (pend) return -1;
-            if ((pit & 1) != dset) {          // the other set's step
+            while (pit % kDecSets != dset) {  // the other sets' steps
                 ++pkt;
                 ++pit;
                 advance();
                 if (pend) return -1;
             }
-            int64_t row = prow[(int64_t)pkt * kBK];
-            // bounds-checked build: a member row outside the image is not gathered
-            if (!in_range(a.m_pad == 0 || (row >= 0 && row < a.m_pad), 0x1001u)) row = -2;
+            const int32_t row = prow[(int64_t)pkt * kBK];
             ++pkt;
             ++pit;
             return row;
         };
         int pslot = dset;                     // ring slot of the step being fetched
-        int64_t row_next = cursor_row();
+        // (kept as loaded: anything computed from it here would wait for the load)
+        int32_t row_next = cursor_row();
         auto prefetch_one = [&]() {
-            const int64_t row = row_next;
+            const int32_t row = row_next;
             row_next = cursor_row();
-            if (row >= 0) {
-                const uint8_t* src = codes + row * a.nbp;
+            // bounds-checked build: a member row outside the image is not gathered
+            if (row >= 0 && in_range(a.m_pad == 0 || row < a.m_pad, 0x1001u)) {
+                const uint8_t* src = codes + (int64_t)row * a.nbp;
                 uint8_t* dst = ring + pslot * kRingSlot + t * 32;
                 cp_async16(dst, src);
                 cp_async16(dst + 16, src + 16);
             }
             cp_async_commit();
-            pslot = pslot + 2 < kRing ? pslot + 2 : dset;
+            pslot = pslot + kDecSets < kRing ? pslot + kDecSets : dset;
         };
-        constexpr int kDepth = kRing / 2;     // steps of this set in flight
         for (int d = 0; d < kDepth - 1; ++d) prefetch_one();
         int it = 0, s = 0, slot = 0;
         uint32_t ph = 0;
@@ -296,22 +311,21 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             int k0;
             const int nkt = steps_of(q, k0) * a.ngroups;
             for (int kt = 0; kt < nkt; ++kt, ++it) {
-                if ((it & 1) == dset) {
+                if (it % kDecSets == dset) {
                     prefetch_one();
                     asm volatile("cp.async.wait_group %0;\n" ::"n"(kDepth - 1));
                     const uint4* src =
                         reinterpret_cast<const uint4*>(ring + slot * kRingSlot + t * 32);
                     const uint4 c0 = src[0], c1 = src[1];
-                    if (it >= nst && !__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1u))) {
+                    if (it >= nst && !warp_wait(&empty[s], ph ^ 1u, abort_flag)) {
                         fail(14);
                         break;
                     }
-                    if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
                     uint8_t* gRow = smem + s * lay.stage + (t >> 3) * 1024 + (t & 7) * 128;
                     decode_row_sw128(c0, c1, gRow, gRow + kATile, t);
                     fence_async_smem();
                     __syncwarp();  // orders the warp's operand stores before its one arrival
-                    if (lane == 0) mbar_arrive(&full_dec[s]);
+                    if (lane == 0) mbar_arrive(&full[s]);
                 }
                 if (++s == nst) { s = 0; ph ^= 1u; }
                 if (++slot == kRing) slot = 0;
@@ -319,18 +333,15 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         }
         cp_async_wait_all();  // no gather copy may outlive the CTA (abort path)
     } else {
-        // ---------------- epilogue (four warps per TMEM lane quadrant) ----------------
-        const int e = tid - 32 * kEpiWarp0;
+        // ---------------- epilogue (eight warps per accumulator) ----------------
+        // Each half of the warps answers for one accumulator, so that the waits,
+        // loads and shuffles of one job overlap the arithmetic of the next.
+        const int half = (warp - kEpiWarp0) / kEpiWarps;
+        const int e = (tid - 32 * kEpiWarp0) % kEpiThreads;
         const int q = warp & 3;                  // TMEM lane quadrant of this warp
-        const int h = (warp - kEpiWarp0) >> 2;   // which quarter of the column chunks
+        const int h = ((warp - kEpiWarp0) >> 2) & 1;  // which of every two column chunks
         const int64_t i = i0 + q * 32 + lane;    // sample row of this thread's accumulator lane
-        int4* const tab = shift_tab + (warp - kEpiWarp0) * 16;   // this warp's digit shifts
-        // The digit shift of probe vl of this warp's (at most two) chunks of 8,
-        // loaded one job ahead.
-        auto load_shift = [&](int k, int g) {
-            const int v = g * 64 + 8 * (h + 4 * ((lane >> 3) & 1)) + (lane & 7);
-            return v < a.V ? a.yshift[(int64_t)k * a.V + v] : 0;
-        };
+        int4* const tab = shift_tab + (warp - kEpiWarp0) * 32;   // this warp's digit shifts
         // Sketch column, counted from the job's first bin, of digit-column group
         // `slot` (4 columns each): -1 past a bin's probes or the job's bins.
         auto probe_of = [&](int slot, int nbin) -> int64_t {
@@ -338,18 +349,21 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             const int per = a.ncolp / 4, u = slot / per, v = slot - u * per;
             return u < nbin && v < a.V ? (int64_t)u * a.V + v : -1;
         };
-        int shift_next = a.yq ? load_shift(kb0, 0) : 0;
         int au = 0;
         for (int kq = 0; kq < nsb && !__any_sync(0xffffffffu, *abort_flag != 0); kq += a.share) {
             const int k = kb0 + kq;
             int k0;
             const int nkt = steps_of(kq, k0), nbin = min(a.share, nsb - kq);
+            if (nkt == 0 ? (au & 1) != half : a.ngroups == 1 && (au & 1) != half) {
+                if (nkt > 0) ++au;
+                continue;
+            }
             // This sample tile's block of super-bin k in phase 2's digit layout
             // (digit_offset): ncolp rows of 128 bytes.
             int8_t* const yblk =
                 a.yq ? a.yq + ((int64_t)blockIdx.x * a.K * a.ncolp + (int64_t)k * a.ncolp) * 128
                      : nullptr;
-            if (a.yq) {
+            if (a.yq && (nkt == 0 || ((au + a.ngroups - 1) & 1) == half)) {
                 // Digit padding rows 4V..ncolp of this tile read as zero in phase 2.
                 for (int idx = e; idx < (a.ncolp - 4 * a.V) * 8; idx += kEpiThreads)
                     *reinterpret_cast<uint4*>(yblk + (4 * a.V + (idx >> 3)) * 128 + (idx & 7) * 16) =
@@ -368,32 +382,32 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                         *reinterpret_cast<uint4*>(a.Y + ((int64_t)k * a.V + (idx >> 6)) * a.N_pad +
                                                   i0 + (idx & 63) * 2) = make_uint4(0, 0, 0, 0);
                 }
-                if (a.yq && kq + 1 < nsb) shift_next = load_shift(k + 1, 0);
                 continue;
             }
             // (nkt is this super-bin's whole list: the digit form is never split)
             const bool small_sums = nkt <= kMaxNarrowSteps;
             for (int g = 0; g < a.ngroups && !__any_sync(0xffffffffu, *abort_flag != 0); ++g, ++au) {
                 const int b = au & 1, u = au >> 1;
+                if (b != half) continue;
                 // Loaded before the accumulator wait so the loads overlap the MMAs:
-                // the digit shifts of this warp's (at most two) chunks of 8 probes,
+                // the digit shifts of this warp's (at most four) chunks of 8 probes,
                 // or the group's 64 per-probe scales, two per lane.
                 bool narrow = false;
                 double scA = 0.0, scB = 0.0;
                 if (a.yq) {
-                    const int r = -shift_next;
+                    const int v = g * 64 + 8 * (h + 2 * (lane >> 3)) + (lane & 7);
+                    const int r = v < a.V ? -a.yshift[(int64_t)k * a.V + v] : 0;
                     narrow = small_sums && __all_sync(0xffffffffu, r >= 0 && r <= 14);
                     // x = right shift, y = 14 - x, z = half an ulp less one, w = parity mask
-                    if (lane < 16)
-                        tab[lane] = make_int4(r, 14 - r, r > 0 ? (1 << ((r - 1) & 15)) - 1 : 0,
-                                              r > 0 ? 1 : 0);
+                    tab[lane] = make_int4(r, 14 - r, r > 0 ? (1 << ((r - 1) & 15)) - 1 : 0,
+                                          r > 0 ? 1 : 0);
                     __syncwarp();
                 } else {
                     const int64_t oa = probe_of(g * 64 + lane, nbin), ob = probe_of(g * 64 + lane + 32, nbin);
                     if (oa >= 0) scA = a.colscale[(int64_t)k * a.V + oa];
                     if (ob >= 0) scB = a.colscale[(int64_t)k * a.V + ob];
                 }
-                if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (uint32_t)u & 1u))) {
+                if (!warp_wait(&acc_full[b], (uint32_t)u & 1u, abort_flag)) {
                     fail(15);
                     break;
                 }
@@ -401,11 +415,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                 const int ncols = min(kAccCols, nbin * a.ncolp - g * 256);
                 const uint32_t tbase = tmem + (uint32_t)(b * kAccCols) + ((uint32_t)(q * 32) << 16);
                 if (a.yq) {
-                    if (g + 1 < a.ngroups) shift_next = load_shift(k, g + 1);
-                    else if (kq + 1 < nsb) shift_next = load_shift(k + 1, 0);
                     // Digits straight into phase 2's operand layout, 8 probes (32
-                    // digit columns) per TMEM load; the quadrant's four warps take
-                    // every fourth chunk.  With y = T 2^(eW-28) and the column
+                    // digit columns) per TMEM load; the quadrant's two warps take
+                    // every second chunk.  With y = T 2^(eW-28) and the column
                     // exponent eY fixed in advance by a bound on |y|, the sketch's
                     // 28-bit value is R = rint(T 2^-r), r = eY - eW (round half to
                     // even), and digits_word splits it.  A 4 x 4 byte transpose
@@ -430,7 +442,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     int8_t* const ylane = yblk + qd * 128 + 4 * ((lane >> 2) & 3);
                     int8_t* const ydst[2] = {ylane + ((chunk ^ qd) << 4),
                                              ylane + ((chunk ^ (4 + qd)) << 4)};
-                    for (int c0 = 32 * h, cc = 0; c0 < ncols; c0 += 128, cc += 8) {
+                    for (int c0 = 32 * h, cc = 0; c0 < ncols; c0 += 64, cc += 8) {
                         int rr[32];
                         tmem_ld32(tbase + (uint32_t)c0, rr);
                         tmem_wait_ld(rr);
@@ -478,7 +490,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                                     w[p];
                     }
                 } else {
-                for (int c0c = 16 * h; c0c < ncols; c0c += 64) {
+                for (int c0c = 16 * h; c0c < ncols; c0c += 32) {
                     int rr[16];
                     tmem_ld16(tbase + (uint32_t)c0c, rr);
                     tmem_wait_ld(rr);
@@ -512,9 +524,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     }
 }
 
-// Weight digits in the layout of p1_umma_kernel:
-// Wq[((k*2 + part)*ncolp + 4 v + t)*Lmax + r], part 0 = W1, 1 = -W2.
-// Entries past a list's padded length are never read.
+// Weight digits in the layout of p1_umma_kernel (w_digit_offset): part 0 = W1,
+// 1 = -W2, column 4 v + t = digit t of probe v.  The padding columns
+// 4V..ncolp are left as they are: their accumulator columns are never read.
 //
 // Latency-bound gathers (rowind -> sdinv, mean, Z) followed by 8 bytes written
 // per (member, probe).  A cluster of CTAs owns a (bin, probe) column: each CTA
@@ -622,8 +634,6 @@ __global__ void __launch_bounds__(kWarp ? 32 * kWWarps : kWMaxThreads)
     // 2^(28 - e) as two factors: it overflows for columns of tiny weights.
     const int e1 = min(28 - e, 1000);
     const double f1 = ldexp(1.0, e1), f2 = ldexp(1.0, 28 - e - e1);
-    int8_t* b1 = w.wq + ((int64_t)(k * 2 + 0) * w.ncolp + 4 * v) * w.lmax;
-    int8_t* b2 = w.wq + ((int64_t)(k * 2 + 1) * w.ncolp + 4 * v) * w.lmax;
     for (int64_t r = rbeg; r < nnzp; r += stride) {
         double a[4], m[4];
         if (r == rbeg) {
@@ -639,15 +649,17 @@ __global__ void __launch_bounds__(kWarp ? 32 * kWWarps : kWMaxThreads)
 #pragma unroll
         for (int q = 0; q < 4; ++q) x[q] = digits_word(__double2int_rn(a[q] * f1 * f2));
         transpose4x4(x[0], x[1], x[2], x[3], d[3], d[2], d[1], d[0]);  // byte b: digit 3 - b
+        const int64_t step = (r0 + r) / kP1Step;
+        const int rs = (int)(r % kP1Step);
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-            *reinterpret_cast<uint32_t*>(b1 + (int64_t)s * w.lmax + r) = d[s];
+        for (int t = 0; t < 4; ++t)
+            *reinterpret_cast<uint32_t*>(w.wq + w_digit_offset(step, 0, 4 * v + t, rs, w.ncolp)) = d[t];
 #pragma unroll
         for (int q = 0; q < 4; ++q) x[q] = digits_word(__double2int_rn(-(m[q] * f1 * f2)));
         transpose4x4(x[0], x[1], x[2], x[3], d[3], d[2], d[1], d[0]);
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-            *reinterpret_cast<uint32_t*>(b2 + (int64_t)s * w.lmax + r) = d[s];
+        for (int t = 0; t < 4; ++t)
+            *reinterpret_cast<uint32_t*>(w.wq + w_digit_offset(step, 1, 4 * v + t, rs, w.ncolp)) = d[t];
     }
     if (rank == 0 && gtid == 0) {
         w.colscale[kv] = ldexp(1.0, e - 7 - 21);
@@ -684,7 +696,8 @@ void launch_p1_weights4(const P1UWeights& w, const double* mean, const double* s
     // cluster where that is more than a CTA's and the columns alone leave SMs
     // without a CTA.
     const int64_t quads = (w.lmax + 3) / 4;
-    const int threads = (int)std::min<int64_t>(kWMaxThreads, (quads + 31) / 32 * 32);
+    const int threads =
+        (int)std::max<int64_t>(32, std::min<int64_t>(kWMaxThreads, (quads + 31) / 32 * 32));
     int width = 1;
     while (width < 8 && kv * width < 2 * 148 && quads > (int64_t)threads * width) width *= 2;
     cudaLaunchConfig_t cfg = {};
@@ -708,7 +721,7 @@ void prepare_p1_umma() {
                          p1::kSmemLimit);
 }
 
-void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cudaStream_t st) {
+void launch_p1_umma(const P1UArgs& a, int64_t N_pad, cudaStream_t st) {
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] { prepare_p1_umma(); });
     P1UArgs b = a;
@@ -724,11 +737,11 @@ void launch_p1_umma(const CUtensorMap& tmW, const P1UArgs& a, int64_t N_pad, cud
     const int64_t ctas = (int64_t)grid.x * grid.y, steps = a.lmax / p1::kBK;
     b.nsplit = 1;
     if (!a.yq && ctas > 0 && a.lmax <= ((int64_t)1 << 22))
-        b.nsplit = (int)std::max<int64_t>(1, std::min<int64_t>(148 / ctas, steps / 8));
+        b.nsplit = (int)std::max<int64_t>(1, std::min<int64_t>(148 / ctas, steps / 16));
     grid.z = (unsigned)b.nsplit;
     if (b.nsplit > 1)
         cudaMemsetAsync(a.Y, 0, sizeof(double) * (size_t)(a.K * a.V) * (size_t)N_pad, st);
-    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(p1_tile_rows(b)), st>>>(tmW, b);
+    p1_umma_kernel<<<grid, p1::kThreads, p1_umma_smem_bytes(p1_tile_rows(b)), st>>>(b);
     count_launch();
 }
 
