@@ -4250,11 +4250,10 @@ void window_ld_impl(Context& c, const Prepared& P, int64_t row0, int64_t row1, c
         lo32[(size_t)r] = (int32_t)std::min(row1, std::max(row0, lo[r]));
         hi32[(size_t)r] = (int32_t)std::min(row1, std::max(row0, hi[r]));
     }
-    constexpr int64_t TB = 128;
+    constexpr int64_t TB = kGramTile;
     const int64_t nT = (m + TB - 1) / TB;
     // Partner tiles of each row tile, on the same 128-grid from row0.
     std::vector<std::pair<int64_t, int64_t>> span((size_t)nT, {0, 0});
-    int64_t pairs = 0;
     for (int64_t T = 0; T < nT; ++T) {
         const int64_t a0 = T * TB, a1 = std::min(m, a0 + TB);
         int64_t lmin = row1, hmax = row0;
@@ -4263,27 +4262,70 @@ void window_ld_impl(Context& c, const Prepared& P, int64_t row0, int64_t row1, c
             lmin = std::min<int64_t>(lmin, lo32[(size_t)r]);
             hmax = std::max<int64_t>(hmax, hi32[(size_t)r]);
         }
-        if (hmax > lmin) {
-            span[(size_t)T] = {(lmin - row0) / TB, (hmax - 1 - row0) / TB + 1};
-            pairs += span[(size_t)T].second - span[(size_t)T].first;
+        if (hmax > lmin) span[(size_t)T] = {(lmin - row0) / TB, (hmax - 1 - row0) / TB + 1};
+    }
+    // Unordered tile pairs (J <= I) that either side needs.
+    std::vector<std::vector<int32_t>> pairs((size_t)nT);
+    int64_t npairs = 0;
+    for (int64_t T = 0; T < nT; ++T)
+        for (int64_t u = span[(size_t)T].first; u < span[(size_t)T].second; ++u)
+            pairs[(size_t)std::min(T, u)].push_back((int32_t)std::max(T, u));
+    for (auto& v : pairs) {
+        std::sort(v.begin(), v.end());
+        v.erase(std::unique(v.begin(), v.end()), v.end());
+        npairs += (int64_t)v.size();
+    }
+    // Partner tiles per CTA: the fewest K-steps on the busiest SM, a CTA's start
+    // and last read-out counted as 12 of them (12,000 SNPs, 1,500 pairs: 1 per CTA,
+    // 11 rounds; 2 would leave the last of 6 rounds nearly empty).
+    const int64_t nkt = P.g.N_pad / 128;
+    int64_t per_cta = 1, best = std::numeric_limits<int64_t>::max();
+    for (int64_t p = 1; p <= 8; ++p) {
+        const int64_t rounds = ((npairs + p - 1) / p + 147) / 148, cost = rounds * (p * nkt + 12);
+        if (cost < best) {
+            best = cost;
+            per_cta = p;
         }
     }
-    const int64_t per_cta = std::max<int64_t>(1, std::min<int64_t>(8, pairs / (148 * 4)));
-    std::vector<int4> items;
-    std::vector<int32_t> slot_beg((size_t)nT + 1, 0);
+    // CTAs (runs of consecutive partner tiles), in batches whose units stay
+    // within 512 MB (at least one CTA each).
+    struct GramBatch {
+        std::vector<GramItem> items;
+        std::vector<std::pair<int32_t, int32_t>> uses;   // (tile, unit)
+        int64_t units = 0;
+    };
+    const int64_t max_units = std::max<int64_t>(1, ((int64_t)512 << 20) / (TB * K * 8));
+    std::vector<GramBatch> batches(1);
     for (int64_t T = 0; T < nT; ++T) {
-        for (int64_t u = span[(size_t)T].first; u < span[(size_t)T].second; u += per_cta)
-            items.push_back(make_int4((int)(row0 + T * TB), (int)(row0 + u * TB),
-                                      (int)std::min(per_cta, span[(size_t)T].second - u),
-                                      (int)items.size()));
-        slot_beg[(size_t)T + 1] = (int32_t)items.size();
+        const std::vector<int32_t>& v = pairs[(size_t)T];
+        for (size_t x = 0; x < v.size();) {
+            size_t y = x + 1;
+            while (y < v.size() && (int64_t)(y - x) < per_cta && v[y] == v[y - 1] + 1) ++y;
+            const int n = (int)(y - x), off = v[x] == T ? n - 1 : n;
+            if (!batches.back().items.empty() && batches.back().units + kGramRowUnits + 4 * off > max_units)
+                batches.emplace_back();
+            GramBatch& b = batches.back();
+            const int32_t ru = (int32_t)b.units, cu = ru + kGramRowUnits;
+            b.items.push_back({(int32_t)(row0 + T * TB), (int32_t)(row0 + v[x] * TB), n, ru, cu});
+            for (int w = 0; w < kGramRowUnits; ++w) b.uses.push_back({(int32_t)T, ru + w});
+            for (int z = 0; z < off; ++z)
+                for (int w = 0; w < 4; ++w)
+                    b.uses.push_back({v[y - (size_t)off + (size_t)z], cu + 4 * z + w});
+            b.units += kGramRowUnits + 4 * off;
+            x = y;
+        }
     }
-    DevBuf d_items, d_beg, d_lo, d_hi, d_mu, d_rs, d_annot, d_part, d_out, d_st;
-    const size_t nit = std::max<size_t>(items.size(), 1);
-    int4* di = d_items.as<int4>(nit);
-    h2d(di, items.data(), items.size(), c.st);
-    int32_t* db = d_beg.as<int32_t>(slot_beg.size());
-    h2d(db, slot_beg.data(), slot_beg.size(), c.st);
+    DevBuf d_items, d_beg, d_list, d_lo, d_hi, d_mu, d_rs, d_annot, d_units, d_out, d_st;
+    int64_t munits = 1;
+    size_t mitems = 1, muses = 1;
+    for (const GramBatch& b : batches) {
+        munits = std::max(munits, b.units);
+        mitems = std::max(mitems, b.items.size());
+        muses = std::max(muses, b.uses.size());
+    }
+    GramItem* di = d_items.as<GramItem>(mitems);
+    int32_t* db = d_beg.as<int32_t>((size_t)nT + 1);
+    int32_t* dl = d_list.as<int32_t>(muses);
     int32_t* dlo = d_lo.as<int32_t>((size_t)m);
     int32_t* dhi = d_hi.as<int32_t>((size_t)m);
     h2d(dlo, lo32.data(), (size_t)m, c.st);
@@ -4294,14 +4336,13 @@ void window_ld_impl(Context& c, const Prepared& P, int64_t row0, int64_t row1, c
     h2d(drs, rs.data(), rs.size(), c.st);
     double* dan = d_annot.as<double>((size_t)(m * K));
     h2d(dan, annot, (size_t)(m * K), c.st);
-    const size_t npart = nit * (size_t)TB * (size_t)K;
-    double* dpart = d_part.as<double>(npart);
-    ck(cudaMemsetAsync(dpart, 0, npart * sizeof(double), c.st), "memset partial");
+    double* dun = d_units.as<double>((size_t)(munits * TB * K));
     double* dout = d_out.as<double>((size_t)(m * K));
+    ck(cudaMemsetAsync(dout, 0, sizeof(double) * (size_t)(m * K), c.st), "memset");
     unsigned* dst = d_st.as<unsigned>(1);
     ck(cudaMemsetAsync(dst, 0, 4, c.st), "memset");
     GramArgs ga;
-    ga.nkt = (int)(P.g.N_pad / 128);
+    ga.nkt = (int)nkt;
     ga.K = (int)K;
     ga.row0 = row0;
     ga.row1 = row1;
@@ -4312,27 +4353,51 @@ void window_ld_impl(Context& c, const Prepared& P, int64_t row0, int64_t row1, c
     ga.rs = drs;
     ga.annot = dan;
     ga.corr_den = corr_dim > 0.0 ? 1.0 / (corr_dim - 1.0) : 0.0;
-    ga.partial = dpart;
+    ga.units = dun;
     ga.status = dst;
     const CUtensorMap tmC = make_map_2d(P.g.codes, (uint64_t)P.g.nbp, (uint64_t)P.g.M_pad,
                                         (uint64_t)P.g.nbp, 32, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
-    ck(cudaEventRecord(c.ev[0], c.st), "event");
-    launch_gram_ld(tmC, ga, (int)items.size(), c.st);
-    ck(cudaEventRecord(c.ev[2], c.st), "event");
-    launch_gram_reduce(dpart, db, row0, row1, (int)K, dout, K, 1, c.st);
-    ck(cudaEventRecord(c.ev[1], c.st), "event");
-    ck(cudaGetLastError(), "launch");
+    double gram_ms = 0.0, total_ms = 0.0;
+    for (GramBatch& b : batches) {
+        // each tile's units in the order they were made
+        std::vector<int32_t> beg((size_t)nT + 1, 0), list(b.uses.size());
+        for (const auto& u : b.uses) ++beg[(size_t)u.first + 1];
+        for (int64_t T = 0; T < nT; ++T) beg[(size_t)T + 1] += beg[(size_t)T];
+        std::vector<int32_t> at(beg.begin(), beg.end() - 1);
+        for (const auto& u : b.uses) list[(size_t)at[(size_t)u.first]++] = u.second;
+        h2d(di, b.items.data(), b.items.size(), c.st);
+        h2d(db, beg.data(), beg.size(), c.st);
+        h2d(dl, list.data(), list.size(), c.st);
+        ck(cudaEventRecord(c.ev[0], c.st), "event");
+        launch_gram_ld(tmC, ga, (int)b.items.size(), c.st);
+        ck(cudaEventRecord(c.ev[2], c.st), "event");
+        launch_gram_reduce(dun, db, dl, row0, row1, (int)K, dout, c.st);
+        ck(cudaEventRecord(c.ev[1], c.st), "event");
+        ck(cudaGetLastError(), "launch");
+        if (batches.size() > 1) {   // the tables are reused by the next batch
+            ck(cudaStreamSynchronize(c.st), "windowed LD batch");
+            float ms = 0.f;
+            ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[1]), "elapsed");
+            total_ms += ms;
+            ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[2]), "elapsed");
+            gram_ms += ms;
+        }
+    }
     std::vector<double> h((size_t)(m * K));
     d2h(h.data(), dout, h.size(), c.st);
     unsigned stv = 0;
     d2h(&stv, dst, 1, c.st);
     ck(cudaStreamSynchronize(c.st), "windowed LD");
     if (stv) fail(LDS_ERR_CUDA, "windowed LD tensor-core pipeline wait timed out (code %u)", stv);
-    float ms = 0.f;
-    ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[1]), "elapsed");
-    c.timings[0] = ms;
-    ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[2]), "elapsed");
-    c.timings[1] = ms;  // Gram kernel alone
+    if (batches.size() == 1) {
+        float ms = 0.f;
+        ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[1]), "elapsed");
+        total_ms = ms;
+        ck(cudaEventElapsedTime(&ms, c.ev[0], c.ev[2]), "elapsed");
+        gram_ms = ms;
+    }
+    c.timings[0] = total_ms;
+    c.timings[1] = gram_ms;  // Gram kernel alone
     for (int64_t r = 0; r < m; ++r)
         for (int64_t b = 0; b < K; ++b) out[r * ld_row + b * ld_col] = h[(size_t)(r * K + b)];
 }

@@ -103,30 +103,37 @@ void launch_nn_band(const DevGeno& g, int D, int32_t* counts, cudaStream_t st);
 void launch_nn_band_finish(int64_t M, int D, const int32_t* counts, const double* mean,
                            const double* sdinv, double* xx, cudaStream_t st);
 
-// Exact windowed LD scores (lds_gram.cu).  Work item x: tile J = SNPs
-// [x.x, x.x + 128), partner tiles I = [x.y + 128 t, +128) for t < x.z, sums
-// into partial slot x.w.  lo/hi: partner interval of SNP j at (j - row0);
-// mean/rs (1/sqrt(c_jj), 0 for a constant SNP) indexed by SNP; annot row-major
-// ((i - row0) K + b); corr_den = 1/(corr_dim - 1) for the unbiased r^2, 0 for r^2.
+// Exact windowed LD scores (lds_gram.cu).  lo/hi: partner interval of SNP j at
+// (j - row0); mean/rs (1/sqrt(c_jj), 0 for a constant SNP) indexed by SNP; annot
+// row-major ((i - row0) K + b); corr_den = 1/(corr_dim - 1) for the unbiased r^2,
+// 0 for r^2.
+constexpr int kGramTile = 128;      // SNPs per tile
+constexpr int kGramRowUnits = 4;    // row-sum units of a work item
+// One CTA's work: tile J (rows jrow0..) against `tiles` partner tiles from irow0
+// on, all at or after J.  Its row sums go to kGramRowUnits units from row_unit on,
+// the column sums of its t-th partner tile other than J itself to the four units
+// from col_unit + 4 t on; a unit is 128 SNPs x K doubles.
+struct GramItem {
+    int32_t jrow0, irow0, tiles, row_unit, col_unit;
+};
 struct GramArgs {
     int nkt = 0, K = 0;
     int64_t row0 = 0, row1 = 0;
-    const int4* items = nullptr;
+    const GramItem* items = nullptr;
     const int32_t* lo = nullptr;
     const int32_t* hi = nullptr;
     const double* mean = nullptr;
     const double* rs = nullptr;
     const double* annot = nullptr;
     double corr_den = 0.0;
-    double* partial = nullptr;      // (slot 128 + jl) K + b, zeroed by the caller
+    double* units = nullptr;
     unsigned* status = nullptr;
 };
-size_t gram_ld_smem_bytes();
 void launch_gram_ld(const CUtensorMap& tmC, const GramArgs& a, int n_items, cudaStream_t st);
-// out[(j - row0) ld_row + b ld_col] = sum of tile (j - row0)/128's slots
-// [slot_beg[T], slot_beg[T+1]) in order.
-void launch_gram_reduce(const double* partial, const int32_t* slot_beg, int64_t row0, int64_t row1,
-                        int K, double* out, int64_t ld_row, int64_t ld_col, cudaStream_t st);
+// out[(j - row0) K + b] += the sum over tile T = (j - row0)/128's units
+// list[beg[T]..beg[T+1]), in order.
+void launch_gram_reduce(const double* units, const int32_t* beg, const int32_t* list, int64_t row0,
+                        int64_t row1, int K, double* out, cudaStream_t st);
 
 // GxE (lds_gxe.cu): see the file header for the column layouts.
 void launch_gxe_source_finalize(const double* Y, int64_t N, int64_t N_pad, int64_t C, int cols_half,

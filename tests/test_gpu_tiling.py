@@ -100,3 +100,32 @@ def test_component_diagonal_forms(oracle, Q, R, K, m):
     go.component_diagonal(X, 0, m, annot, basis, fixed, coef, want)
     assert rel_err(got, want) < 1e-12   # FP64 sums of at most 200 terms
     sess.close()
+
+
+# Unordered tile pairs: one tile; a ragged last tile; runs of several tiles per
+# CTA (many pairs); one-sided and empty partner intervals, which the two orders of
+# a pair see differently; K over one pass of 8, at 4 and at 1; a sub-range.
+@pytest.mark.parametrize("n,m,K,reach,row0", [(300, 100, 1, 30, 0), (200, 700, 3, 260, 0),
+                                              (40, 6000, 2, 5999, 0), (257, 500, 9, 200, 37),
+                                              (130, 400, 4, 400, 0)])
+def test_window_ld_pairs(oracle, n, m, K, reach, row0):
+    from oracle.oracle import windowed_ld_exact
+    from summit_b200.session import GwSession
+
+    rng = np.random.default_rng(m)
+    rows = _rows(n, m, seed=K)
+    X = oracle.standardize(rows, n, 0, m)[0]
+    mm = m - row0
+    j = np.arange(mm)
+    lo, hi = np.maximum(0, j - reach), np.minimum(mm, j + reach + 1)
+    odd = rng.random(mm) < 0.3
+    lo[odd] = j[odd]                 # these look only to the right
+    hi[::7] = lo[::7]                # and these have no partner
+    annot = rng.random((mm, K))
+    sess = GwSession(rows, n)
+    got = sess.window_ld(lo + row0, hi + row0, annot, corr_dim=n - 1.0, row0=row0)
+    again = sess.window_ld(lo + row0, hi + row0, annot, corr_dim=n - 1.0, row0=row0)
+    np.testing.assert_array_equal(got, again)
+    ref = windowed_ld_exact(X[:, row0:], annot, lo, hi, restandardize=True, corr_dim=n - 1.0)
+    assert rel_err(got, ref) < 1e-11   # integer Gram sums, FP64 after them
+    sess.close()
