@@ -25,8 +25,8 @@
 //
 // Bound by shared-memory bandwidth: per K-step 96 KB of MMA operand reads, 64 KB
 // of decoded operands and 16 KB of packed rows are 1,375 cycles at 128 bytes each
-// (MMA 1,024); it takes about 1,550.  N = 50,000, 12,000 SNPs with partners 2,000
-// to each side: 7.54 -> 3.42 ms (before: both orders of every pair, and four
+// (MMA 1,024); it takes about 1,650.  N = 50,000, 12,000 SNPs with partners 2,000
+// to each side: 7.54 -> 3.6 ms (before: both orders of every pair, and four
 // decoding warps for 256 operand rows).
 //
 // Roles (576 threads): warp 0 TMEM allocation and MMA issue (the warp walks the
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);  // (a plain offset keeps shared-space accesses)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + bar_off());
     uint64_t* pk_full = bars;                    // [kPk] packed rows landed (TMA)
-    uint64_t* pk_empty = pk_full + kPk;          // [kPk] packed rows read by the decoders
+    uint64_t* pk_empty = pk_full + kPk;          // [kPk] packed rows used by the decoders
     uint64_t* full = pk_empty + kPk;             // [kStages] operands decoded
     uint64_t* empty = full + kStages;            // [kStages] operands consumed by the MMAs
     uint64_t* acc_full = empty + kStages;        // accumulators hold a finished tile pair
@@ -217,10 +217,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                     php ^= 1u;
                     const uint4 p0 = pk[0], p1 = pk[1];
                     // The slot goes back as soon as the rows are in registers: the
-                    // vote needs every lane's words, so no read can still be on its way.
-                    const uint32_t all = p0.x & p0.y & p0.z & p0.w & p1.x & p1.y & p1.z & p1.w;
-                    const int seen = __any_sync(0xffffffffu, all == 0x12345678u);
-                    if (lane == 0 && seen >= 0) mbar_arrive(&pk_empty[group]);
+                    // arrival depends on the words that were read (a copy of them
+                    // that the compiler cannot know to be equal), so no read of the
+                    // slot can still be on its way.
+                    const uint32_t words = p0.x ^ p0.y ^ p0.z ^ p0.w ^ p1.x ^ p1.y ^ p1.z ^ p1.w;
+                    uint32_t same;
+                    asm volatile("shfl.sync.bfly.b32 %0, %1, 0, 31, 0xffffffff;"
+                                 : "=r"(same)
+                                 : "r"(words));
+                    __syncwarp();
+                    if (lane == 0 && same == words) mbar_arrive(&pk_empty[group]);
                     if (it >= kStages && !warp_wait(&empty[s], ph ^ 1u, abort_flag)) {
                         fail(35);
                         break;

@@ -107,7 +107,7 @@ def test_component_diagonal_forms(oracle, Q, R, K, m):
 # a pair see differently; K over one pass of 8, at 4 and at 1; a sub-range.
 @pytest.mark.parametrize("n,m,K,reach,row0", [(300, 100, 1, 30, 0), (200, 700, 3, 260, 0),
                                               (40, 6000, 2, 5999, 0), (257, 500, 9, 200, 37),
-                                              (130, 400, 4, 400, 0)])
+                                              (130, 400, 4, 400, 0), (30000, 520, 2, 300, 0)])
 def test_window_ld_pairs(oracle, n, m, K, reach, row0):
     from oracle.oracle import windowed_ld_exact
     from summit_b200.session import GwSession
