@@ -242,7 +242,7 @@ struct Context {
     DevBuf colsum;  // per-block phase 2: sketch digit column sums (images with complete tiles)
     // Surrogate-network workspace, grow-only so that repeated training and
     // inference calls make no device allocations (cudaFree synchronizes).
-    DevBuf mlp_m, mlp_v, mlp_g, mlp_zs, mlp_dzs, mlp_dout, mlp_rows, mlp_loss, mlp_pack;
+    DevBuf mlp_m, mlp_v, mlp_g, mlp_zs, mlp_dzs, mlp_hs, mlp_dout, mlp_rows, mlp_loss, mlp_pack;
     // Sketch-digit (0) and weight-digit (1) workspaces shared by windowed plans:
     // grow-only, and each plan keeps the buffer its graph captured alive, so
     // creating and destroying plans does not allocate and free gigabytes.
@@ -5142,6 +5142,7 @@ LDS_API int lds_mlp_loss_grad(const float* d_params, int in_dim, int out_dim, co
         const int64_t P = mlp_layout(in_dim, out_dim).total;
         float* z = c.mlp_zs.as<float>((size_t)(n * 3 * kMlpHidden));
         float* dz = c.mlp_dzs.as<float>((size_t)(n * 3 * kMlpHidden));
+        void* hs = c.mlp_hs.as<uint16_t>((size_t)(n * 3 * kMlpHidden));
         float* d = c.mlp_dout.as<float>((size_t)(n * op));
         double* l = c.mlp_loss.as<double>(1);
         ck(cudaMemsetAsync(l, 0, sizeof(double), c.st), "memset");
@@ -5150,7 +5151,7 @@ LDS_API int lds_mlp_loss_grad(const float* d_params, int in_dim, int out_dim, co
         launch_mlp_pack(a, pack, c.st);
         launch_mlp_forward(a, pack, d_x, nullptr, n, d_t, nullptr, z, d, l,
                            1.0f / (float)(n * out_dim), c.st);
-        launch_mlp_backward(a, pack, d_x, nullptr, n, z, d, dz, d_grad, c.st);
+        launch_mlp_backward(a, pack, d_x, nullptr, n, z, d, dz, hs, d_grad, c.st);
         ck(cudaGetLastError(), "launch");
         if (loss_out) d2h(loss_out, l, 1, c.st);
         ck(cudaStreamSynchronize(c.st), "mlp grad");
@@ -5178,6 +5179,7 @@ LDS_API int lds_mlp_train(float* d_params, int in_dim, int out_dim, const float*
         float* dg = c.mlp_g.as<float>((size_t)P);
         float* z = c.mlp_zs.as<float>((size_t)(B * 3 * kMlpHidden));
         float* dz = c.mlp_dzs.as<float>((size_t)(B * 3 * kMlpHidden));
+        void* hs = c.mlp_hs.as<uint16_t>((size_t)(B * 3 * kMlpHidden));
         float* d = c.mlp_dout.as<float>((size_t)(B * op));
         double* l = c.mlp_loss.as<double>((size_t)std::max(epochs, 1));
         ck(cudaMemsetAsync(dm, 0, sizeof(float) * (size_t)P, c.st), "memset");
@@ -5205,7 +5207,7 @@ LDS_API int lds_mlp_train(float* d_params, int in_dim, int out_dim, const float*
                 launch_mlp_pack(a, pack, c.st);
                 launch_mlp_forward(a, pack, d_x, re + s * B, nb, d_t, nullptr, z, d, l + e,
                                    1.0f / (float)(nb * out_dim * nsteps), c.st);
-                launch_mlp_backward(a, pack, d_x, re + s * B, nb, z, d, dz, dg, c.st);
+                launch_mlp_backward(a, pack, d_x, re + s * B, nb, z, d, dz, hs, dg, c.st);
                 ++step;
                 // The loss scale folds 1/nsteps into the gradient (so the epoch's
                 // loss sums to its mean); Adam is invariant to that scale except

@@ -301,8 +301,8 @@ void launch_mlp_forward(const MlpArgs& a, const void* pack, const float* x, cons
                         double* loss, float gscale, cudaStream_t st);
 // Backward: grad (zeroed by the caller) += d loss / d params.
 void launch_mlp_backward(const MlpArgs& a, const void* pack, const float* x, const int32_t* rows,
-                         int64_t n, const float* zs, const float* dout, float* dzs, float* grad,
-                         cudaStream_t st);
+                         int64_t n, const float* zs, const float* dout, float* dzs, void* hs,
+                         float* grad, cudaStream_t st);
 void launch_mlp_adam(float* p, float* m, float* v, const float* g, int64_t P, float lr, float b1,
                      float b2, float eps, float bc1, float bc2, cudaStream_t st);
 

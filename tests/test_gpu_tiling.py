@@ -129,3 +129,37 @@ def test_window_ld_pairs(oracle, n, m, K, reach, row0):
     ref = windowed_ld_exact(X[:, row0:], annot, lo, hi, restandardize=True, corr_dim=n - 1.0)
     assert rel_err(got, ref) < 1e-11   # integer Gram sums, FP64 after them
     sess.close()
+
+
+# (n_in, n_out, n): the forward with several row tiles per CTA (with and without a
+# last partial one, and at the widest layers, where shared memory holds fewer
+# groups), the weight gradient with several 64-row chunks per split.  Loss and
+# gradient in norm, at the network's own tolerance: BF16 operands against an oracle
+# that rounds as the kernels do.
+@pytest.mark.parametrize("n_in,n_out,n", [(5, 2, 148 * 32 + 1), (128, 64, 19000), (33, 17, 38912)])
+def test_network_forms(n_in, n_out, n):
+    import torch
+
+    from oracle import mlp_oracle as mo
+    from summit_b200.surrogate import Surrogate
+
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(n, n_in)).astype(np.float32)
+    t = rng.normal(size=(n, n_out)).astype(np.float32)
+    p = mo.init_params(n_in, n_out, 3)
+    p += rng.normal(0, 0.02, p.size).astype(np.float32)
+    net = Surrogate(n_in, n_out, params=p)
+    xt, tt = torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()
+    x64, t64, p64 = x.astype(np.float64), t.astype(np.float64), p.astype(np.float64)
+    # a row's result does not depend on the launch: pieces of one tile per CTA agree
+    parts = torch.cat([net.forward(xt[i:i + 4736]) for i in range(0, n, 4736)])
+    assert torch.equal(net.forward(xt), parts)
+    loss, g = net.loss_grad(xt, tt)
+    want_loss, want_g = mo.loss_grad(p64, x64, t64, n_in, n_out)
+    assert abs(loss - want_loss) <= 1e-4 * want_loss
+    g = g.cpu().numpy().astype(np.float64)
+    L = mo.layout(n_in, n_out)
+    for k in ["W1", "b1", "W2", "b2", "W3", "b3", "W4", "b4"]:
+        off, m = L[k]
+        err = np.linalg.norm(g[off:off + m] - want_g[off:off + m])
+        assert err <= 2e-3 * max(np.linalg.norm(want_g[off:off + m]), 1e-30), k
