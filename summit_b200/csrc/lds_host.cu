@@ -98,6 +98,9 @@ struct PoolScope {
     ~PoolScope() { t_pool = saved; }
 };
 
+// The pool of buffers that live for one call (CallScope); null until first used.
+cudaMemPool_t g_call_pool = nullptr;
+
 struct DevBuf {
     void* p = nullptr;
     size_t n = 0;
@@ -130,7 +133,14 @@ struct DevBuf {
             ck(cudaMallocFromPoolAsync(&p, bytes, t_pool.pool, t_pool.st), "pool allocation");
             pool_st = t_pool.st;
         } else {
-            ck(cudaMalloc(&p, bytes), "cudaMalloc");
+            cudaError_t e = cudaMalloc(&p, bytes);
+            if (e == cudaErrorMemoryAllocation && g_call_pool) {  // give back what it holds unused
+                cudaGetLastError();
+                cudaDeviceSynchronize();
+                cudaMemPoolTrimTo(g_call_pool, 0);
+                e = cudaMalloc(&p, bytes);
+            }
+            ck(e, "cudaMalloc");
         }
         n = bytes;
         return p;
@@ -147,6 +157,16 @@ struct DevBuf {
         pool_st = nullptr;
     }
     ~DevBuf() { release(); }
+};
+
+// A buffer kept from call to call: ordinary device memory in every scope.
+struct KeptBuf : DevBuf {
+    void* get(size_t bytes) {
+        PoolScope plain(nullptr, nullptr);
+        return DevBuf::get(bytes);
+    }
+    template <typename T>
+    T* as(size_t count) { return static_cast<T*>(get(count * sizeof(T))); }
 };
 
 template <typename T>
@@ -230,7 +250,7 @@ struct Context {
     cudaEvent_t ev[8];
     unsigned* checked_err = nullptr;  // bounds-checked build: first failed index check
     std::list<std::unique_ptr<Prepared>> cache;  // most recent first
-    DevBuf raw, rows_dev, hwe_q0, hwe_q01, hwe_sb, counts_dev, units_dev;
+    KeptBuf raw, rows_dev, hwe_q0, hwe_q01, hwe_sb, counts_dev, units_dev;
     // Image preparation stream of the streamed one-call windowed estimate
     // (highest priority, so its short kernels are scheduled between the
     // estimate's CTAs), and a grow-only pinned staging area for its results.
@@ -238,11 +258,16 @@ struct Context {
     cudaMemPool_t pool = nullptr;   // chunk images and plans (PoolScope on st_prep)
     void* pinned = nullptr;
     size_t pinned_n = 0;
-    DevBuf y, yq, ycs, wq, wcs, z, rowind, sc, binoff, wqoff, accum, mc, guards, lscale, xin;
-    DevBuf colsum;  // per-block phase 2: sketch digit column sums (images with complete tiles)
+    // Two pinned halves through which the per-block calls' sketches cross PCIe
+    // (kStageBytes each, or one column where that is longer), and their events.
+    void* stage = nullptr;
+    size_t stage_n = 0;
+    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    KeptBuf y, yq, ycs, wq, wcs, z, rowind, sc, binoff, wqoff, accum, mc, guards, lscale, xin;
+    KeptBuf colsum;  // per-block phase 2: sketch digit column sums (images with complete tiles)
     // Surrogate-network workspace, grow-only so that repeated training and
     // inference calls make no device allocations (cudaFree synchronizes).
-    DevBuf mlp_m, mlp_v, mlp_g, mlp_zs, mlp_dzs, mlp_hs, mlp_dout, mlp_rows, mlp_loss, mlp_pack;
+    KeptBuf mlp_m, mlp_v, mlp_g, mlp_zs, mlp_dzs, mlp_hs, mlp_dout, mlp_rows, mlp_loss, mlp_pack;
     // Sketch-digit (0) and weight-digit (1) workspaces shared by windowed plans:
     // grow-only, and each plan keeps the buffer its graph captured alive, so
     // creating and destroying plans does not allocate and free gigabytes.
@@ -274,6 +299,114 @@ void ensure_device(Context& c) {
     for (CheckedErrSetter f : checked_err_setters()) ck(f(c.checked_err), "checked error word");
 #endif
     c.ready = true;
+}
+
+// Device buffers made while it is alive come from the library's pool of per-call
+// memory, ordered on the library stream (on which all of a call's work runs), and
+// go back to it.  cudaMalloc and cudaFree take 50 to 100 us each here and the
+// latter waits for the whole device: the 36 pairs of the generalized estimator
+// (4,000 samples, 6,000 SNPs) were 5 of its 7.8 ms, the 19 of a one-call estimate
+// (1,003 samples, 2,001 SNPs) half of its 1.1 ms.  The pool keeps at most
+// kCallPoolKeep unused across calls; lds_clear_device_cache and a failing
+// allocation give that back too.  The scope ends with the stream idle, so that a
+// call that failed leaves no copy from the caller's memory in flight.
+constexpr uint64_t kCallPoolKeep = 512ull << 20;
+
+cudaMemPool_t call_pool(Context& c) {
+    if (!g_call_pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c.device;
+        cudaMemPool_t pool = nullptr;
+        ck(cudaMemPoolCreate(&pool, &props), "memory pool");
+        uint64_t keep = kCallPoolKeep;
+        ck(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "pool attr");
+        g_call_pool = pool;
+    }
+    return g_call_pool;
+}
+
+struct CallScope {
+    cudaStream_t st;
+    PoolScope scope;
+    explicit CallScope(Context& c) : st(c.st), scope(call_pool(c), c.st) {}
+    ~CallScope() { cudaStreamSynchronize(st); }
+};
+
+// ---------------------------------------------------------------------------
+// Columns of doubles between a device array (ld >= rows) and host code that
+// converts or merges them, in pieces of whole columns through pinned memory, so
+// that one piece crosses PCIe while the host works on the other.  The per-block
+// calls (5,000 samples, 4,000 SNPs, K = 2, B = 20: 8 calls of 1.6 MB) moved a
+// column per copy through pageable memory: 8.2 -> 5.1 ms in all.
+// ---------------------------------------------------------------------------
+constexpr size_t kStageBytes = 2ull << 20;
+
+double* stage_half(Context& c, int h, int64_t rows, int64_t* cols_per_piece) {
+    const size_t col = sizeof(double) * (size_t)std::max<int64_t>(rows, 1);
+    const size_t half = std::max(kStageBytes, col);
+    for (cudaEvent_t& e : c.stage_ev)
+        if (!e) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    if (c.stage_n < 2 * half) {
+        ck(cudaStreamSynchronize(c.st), "staging");
+        if (c.stage) cudaFreeHost(c.stage);
+        c.stage = nullptr;
+        c.stage_n = 0;
+        ck(cudaHostAlloc(&c.stage, 2 * half, cudaHostAllocDefault), "pinned staging");
+        c.stage_n = 2 * half;
+    }
+    *cols_per_piece = std::max<int64_t>(1, (int64_t)(half / col));
+    return reinterpret_cast<double*>(static_cast<char*>(c.stage) + (size_t)h * (c.stage_n / 2));
+}
+
+// use(q0, n, p): columns [q0, q0 + n) at p, `rows` apart, in order.
+template <typename F>
+void download_cols(Context& c, const double* d, int64_t ld, int64_t rows, int64_t cols, F&& use) {
+    int64_t per = 1;
+    stage_half(c, 0, rows, &per);
+    const int64_t pieces = (cols + per - 1) / per;
+    auto fetch = [&](int64_t i) {
+        const int64_t q0 = i * per, n = std::min(per, cols - q0);
+        ck(cudaMemcpy2DAsync(stage_half(c, (int)(i & 1), rows, &per), sizeof(double) * (size_t)rows,
+                             d + q0 * ld, sizeof(double) * (size_t)ld,
+                             sizeof(double) * (size_t)rows, (size_t)n, cudaMemcpyDeviceToHost, c.st),
+           "D2H");
+        ck(cudaEventRecord(c.stage_ev[i & 1], c.st), "event");
+    };
+    for (int64_t i = 0; i < std::min<int64_t>(2, pieces); ++i) fetch(i);
+    for (int64_t i = 0; i < pieces; ++i) {
+        ck(cudaEventSynchronize(c.stage_ev[i & 1]), "download");
+        const int64_t q0 = i * per;
+        use(q0, std::min(per, cols - q0),
+            static_cast<const double*>(stage_half(c, (int)(i & 1), rows, &per)));
+        if (i + 2 < pieces) fetch(i + 2);
+    }
+}
+
+// Columns h (T, `rows` apart) to d as FP64, rows..ld of each column zero.
+template <typename T>
+void upload_cols(Context& c, double* d, int64_t ld, const T* h, int64_t rows, int64_t cols) {
+    if (cols <= 0) return;
+    if (ld > rows)
+        ck(cudaMemset2DAsync(d + rows, sizeof(double) * (size_t)ld, 0,
+                             sizeof(double) * (size_t)(ld - rows), (size_t)cols, c.st),
+           "memset");
+    int64_t per = 1;
+    stage_half(c, 0, rows, &per);
+    ck(cudaStreamSynchronize(c.st), "staging");   // an earlier call's copies from the halves
+    const int64_t pieces = (cols + per - 1) / per;
+    for (int64_t i = 0; i < pieces; ++i) {
+        const int64_t q0 = i * per, n = std::min(per, cols - q0);
+        double* p = stage_half(c, (int)(i & 1), rows, &per);
+        if (i >= 2) ck(cudaEventSynchronize(c.stage_ev[i & 1]), "upload");
+        for (int64_t x = 0; x < n * rows; ++x) p[x] = (double)h[q0 * rows + x];
+        ck(cudaMemcpy2DAsync(d + q0 * ld, sizeof(double) * (size_t)ld, p,
+                             sizeof(double) * (size_t)rows, sizeof(double) * (size_t)rows, (size_t)n,
+                             cudaMemcpyHostToDevice, c.st),
+           "H2D");
+        ck(cudaEventRecord(c.stage_ev[i & 1], c.st), "event");
+    }
 }
 
 // Mean and inverse sd over observed calls (genotype.cpp:651-689).
@@ -1579,27 +1712,26 @@ void phase1_bed_impl(const char* bed_prefix, const char* fam_path, int blk_start
         project_cols(c, static_cast<double*>(c.y.p), P.g.N_pad, K * v_count, cv, false, tmp);
     }
     // Download the block's contribution and merge with beta semantics.
-    std::vector<double> D((size_t)(N * K * v_count));
-    const double* Y = static_cast<double*>(c.y.p);
-    for (int64_t q = 0; q < K * v_count; ++q)
-        d2h(D.data() + q * N, Y + q * P.g.N_pad, (size_t)N, c.st);
-    ck(cudaStreamSynchronize(c.st), "phase1");
+    std::vector<char> touched((size_t)K, 0), beta1((size_t)K, 1);
     for (int64_t k = 0; k < K; ++k) {
         if (csr.nnz[(size_t)k] == 0) continue;
-        bool beta1 = true;
-        if (bin_init) {
-            beta1 = bin_init[k] != 0;
-            bin_init[k] = 1;
-        }
-        for (int64_t cc = 0; cc < v_count; ++cc) {
-            T* dst = Xz + (k * v_count + cc) * N;
-            const double* src = D.data() + (k * v_count + cc) * N;
-            if (beta1)
+        touched[(size_t)k] = 1;
+        if (bin_init) beta1[(size_t)k] = bin_init[k] != 0;
+    }
+    download_cols(c, static_cast<const double*>(c.y.p), P.g.N_pad, N, K * v_count,
+                  [&](int64_t q0, int64_t nq, const double* p) {
+        for (int64_t q = q0; q < q0 + nq; ++q) {
+            if (!touched[(size_t)(q / v_count)]) continue;
+            T* dst = Xz + q * N;
+            const double* src = p + (q - q0) * N;
+            if (beta1[(size_t)(q / v_count)])
                 for (int64_t n = 0; n < N; ++n) dst[n] = (T)((double)dst[n] + src[n]);
             else
                 for (int64_t n = 0; n < N; ++n) dst[n] = (T)src[n];
         }
-    }
+    });
+    for (int64_t k = 0; bin_init && k < K; ++k)
+        if (touched[(size_t)k]) bin_init[k] = 1;
 }
 
 template <typename T>
@@ -1632,11 +1764,8 @@ void phase2_bed_impl(const char* bed_prefix, const char* fam_path, int blk_start
     if (K > 512) fail(LDS_ERR_ARG, "B too large for fixed seg buffers in phase2_accum_XtXz_bed");
     const int64_t N = P.g.N, Np = P.g.N_pad;
     // Sketch to device (FP64, padded rows zero).
-    std::vector<double> y((size_t)(Np * Q), 0.0);
-    for (int64_t q = 0; q < Q; ++q)
-        for (int64_t n = 0; n < N; ++n) y[(size_t)(q * Np + n)] = (double)Xz[q * N + n];
     double* dY = c.y.as<double>((size_t)(Np * Q));
-    h2d(dY, y.data(), y.size(), c.st);
+    upload_cols<T>(c, dY, Np, Xz, N, Q);
     if (Cm && Rm && p > 0) {
         // Work = ((I - C R) X)^T Xz = X^T (I - C R)^T Xz for the dense form
         // (gwldcore.cpp:2376-2390); the Mailman form projects the sketch,
@@ -3452,6 +3581,9 @@ std::unique_ptr<GxePair> gxe_pair_impl(Context& c, const GxeCtx& g, const double
     pr->N = N;
     pr->C = C;
     pr->G = G;
+    // (the pair's own buffers too: it is made and destroyed once per estimate,
+    // and its destruction waits for the stream)
+    CallScope scope(c);
     DevBuf tr, tw;
     const double* dr = dev_in(c, tr, right, (size_t)(N * C), device_ptrs);
     const double* dw = dev_in(c, tw, w, (size_t)(N * G), device_ptrs);
@@ -3492,6 +3624,7 @@ void gxe_target_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, GxePair& pr,
     const int64_t Kp = 2 * T * 2 * K;
     const int nc = umma::ncolp_for((int)B);
     if (!dense && pr.B != (int)B) {
+        PoolScope scope(call_pool(c), c.st);
         int8_t* yq = pr.yq.as<int8_t>((size_t)(Kp * nc * Np));
         umma::launch_quantize_y4(static_cast<double*>(pr.ypair.p), N, Np, (int)Kp, (int)B, nc, yq,
                                  pr.ycs.as<double>((size_t)(Kp * B)), c.st);
@@ -3651,6 +3784,7 @@ void gw_ldscore_impl(const uint8_t* bed_rows, int64_t row_bytes, int64_t n_total
     if (row_bytes < (n_total + 3) / 4) fail(LDS_ERR_ARG, "bed_row_bytes smaller than ceil(N/4)");
     if (impute != LDS_IMPUTE_MEAN && impute != LDS_IMPUTE_HWE)
         fail(LDS_ERR_ARG, "impute_mode must be 'mean' or 'hwe'");
+    CallScope scope(c);
     ck(cudaEventRecord(c.ev[0], c.st), "event");
     std::shared_ptr<Prepared> P(prepare(c, bed_rows, row_bytes, n_total, M, row_sel, n_sel, impute,
                                         iseed, ddof, "session"));
@@ -3816,9 +3950,16 @@ LDS_API void lds_clear_device_cache(void) {
         cudaDeviceSynchronize();
         cudaMemPoolTrimTo(c.pool, 0);
     }
+    if (g_call_pool) {
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(g_call_pool, 0);
+    }
     if (c.pinned) cudaFreeHost(c.pinned);
     c.pinned = nullptr;
     c.pinned_n = 0;
+    if (c.stage) cudaFreeHost(c.stage);
+    c.stage = nullptr;
+    c.stage_n = 0;
 }
 
 #define P1_ARGS(T)                                                                              \
@@ -4315,6 +4456,7 @@ void window_ld_impl(Context& c, const Prepared& P, int64_t row0, int64_t row1, c
             x = y;
         }
     }
+    CallScope scope(c);
     DevBuf d_items, d_beg, d_list, d_lo, d_hi, d_mu, d_rs, d_annot, d_units, d_out, d_st;
     int64_t munits = 1;
     size_t mitems = 1, muses = 1;
@@ -4428,6 +4570,7 @@ static void window_ld_cov_impl(Context& c, const Prepared& P, int64_t row0, int6
     const int64_t m = row1 - row0, N = P.g.N;
     if (K > window_cov_max_bins())
         fail(LDS_ERR_ARG, "at most %d annotation columns with covariates", window_cov_max_bins());
+    CallScope scope(c);
     DevBuf dann, dlo, dhi, dout, dX, dS, dtmp;
     double* an = dann.as<double>((size_t)(m * K));
     h2d(an, annot, (size_t)(m * K), c.st);
@@ -5532,6 +5675,7 @@ LDS_API int lds_global_variant_probes(uint64_t root_seed, uint64_t namespace_key
             return v ^ (v >> 31);
         };
         const uint64_t root_state = mix(root_seed ^ namespace_key ^ 0x9E3779B97F4A7C15ULL);
+        CallScope scope(c);
         DevBuf d;
         double* dp = d.as<double>((size_t)(L * B));
         launch_global_probes(root_state, v0, L, p0, B, dp, c.st);
@@ -5557,6 +5701,7 @@ LDS_API int lds_generalized_component_diagonal(int64_t geno, int64_t j0, int64_t
         Prepared& P = product_image(geno, j0, j1, 1);
         const int64_t L = j1 - j0, N = P.g.N;
         const int C = K * (Q * (Q + 1) / 2);   // components
+        CallScope scope(c);
         DevBuf da, db, df, dc, dp, dn;
         double* a = da.as<double>((size_t)(L * K));
         double* b = db.as<double>((size_t)(N * Q));
@@ -5611,6 +5756,7 @@ static void gen_pass2_run(Context& c, int64_t geno,
         constexpr int kV2 = 64;
         const int K2 = (cols + kV2 - 1) / kV2, nc = umma::ncolp_for(kV2);
         const int64_t ld = (int64_t)K2 * kV2;
+        CallScope scope(c);
         DevBuf dY, dyq, dcs, dann, dto, df1, df2, ddir, drg, dro, drows, dpart, dst;
         double* Y = dY.as<double>((size_t)(Np * ld));
         ck(cudaMemsetAsync(Y, 0, sizeof(double) * (size_t)(Np * ld), c.st), "memset");
@@ -5709,6 +5855,7 @@ LDS_API int lds_generalized_project(const double* base, const double* basis, con
             R < 0 || R > kGenMaxR || N <= 0)
             fail(LDS_ERR_ARG, "invalid generalized projection arguments");
         const int64_t rows = (int64_t)K * Q * B;
+        CallScope scope(c);
         DevBuf dbase, dbasis, dfixed, dout, dleak, dpn;
         double* db = dbase.as<double>((size_t)((int64_t)K * B * N));
         h2d(db, base, (size_t)((int64_t)K * B * N), c.st);
@@ -5766,6 +5913,8 @@ LDS_API int lds_generalized_pass2_sources(int64_t geno, const double* sources, i
         for (int f = 0; f < F; ++f)
             if (fam_t[f] < 0 || fam_t[f] >= Q || fam_s[f] < 0 || fam_s[f] >= Q)
                 fail(LDS_ERR_ARG, "family basis index out of range");
+        ensure_device(c);
+        CallScope scope(c);   // (before the buffers that `fill` makes)
         DevBuf dS, dbasis, dft, dfs;
         gen_pass2_run(
             c, geno,

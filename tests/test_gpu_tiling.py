@@ -131,6 +131,50 @@ def test_window_ld_pairs(oracle, n, m, K, reach, row0):
     sess.close()
 
 
+# The per-block calls' sketch crosses PCIe in pieces of whole columns: 300,007
+# samples make a column longer than a piece, 60,001 ones several pieces of four
+# columns with a last partial one; a second block merges into the first's.
+@pytest.mark.parametrize("n,m,K,B", [(300007, 24, 1, 3), (60001, 30, 2, 5)])
+def test_block_call_pieces(oracle, tmp_path, n, m, K, B):
+    from summit_b200 import bedfile, gwldcore
+
+    rows = _rows(n, m, seed=n)
+    prefix = bedfile.write_plink(tmp_path / "p", packed=rows, n=n)
+    annot = np.ones((m, K))
+    annot[::3, 1:] = 0.0
+    step = m // 2
+    xz = np.full((n, K * B), np.nan, order="F")   # (the first block overwrites)
+    init, inv, meansq = np.zeros(K, dtype=np.uint8), np.empty(m), np.zeros((m, K))
+    for a in range(0, m, step):
+        e = min(m, a + step)
+        gwldcore.phase1_compute_Xz_bed_chunk(
+            prefix, prefix + ".fam", a, e, annot_blk=annot[a:e], inv_right=inv[a:e], v_start=0,
+            v_count=B, kmax_hint=e - a, seed=9, Xz2d_chunk=xz, bin_init_mask=init, inv_out=inv[a:e],
+            impute_mode="mean")
+    for a in range(0, m, step):
+        e = min(m, a + step)
+        gwldcore.phase2_accum_XtXz_bed(prefix, prefix + ".fam", a, e, inv_left=inv[a:e], tile_nvecs=B,
+                                       Xz2d=xz, meansq_accum=meansq, N_denom=n, impute_mode="mean")
+    ref = oracle.gw_ldscore(rows, n, annot, nvecs=B, step=step, seed=9)
+    assert rel_err(meansq, ref["meansq_accum"]) < TOL
+
+
+# One-call estimates take their buffers from a pool: what an earlier call of
+# another size left in them, or the pool having been emptied, changes no bit.
+def test_one_call_buffers_are_reused():
+    from summit_b200 import _lib, gwldcore
+
+    def run(n, m):
+        r = gwldcore.gw_ldscore(_rows(n, m, seed=n), n, np.ones((m, 2)), 6, 100, 3)
+        return np.array(r["ldscore"])
+
+    first = run(300, 200)
+    run(1500, 700)
+    np.testing.assert_array_equal(run(300, 200), first)
+    _lib.load().lds_clear_device_cache()
+    np.testing.assert_array_equal(run(300, 200), first)
+
+
 # (n_in, n_out, n): the forward with several row tiles per CTA (with and without a
 # last partial one, and at the widest layers, where shared memory holds fewer
 # groups), the weight gradient with several 64-row chunks per split.  Loss and
