@@ -66,9 +66,9 @@ void launch_cv_near(const CvNearArgs& a, int D, cudaStream_t st) {
     count_launch();
 }
 
-// Finalize of a windowed estimate: meansq = sum of the probe slices and
-// ld = meansq / nvecs - Mkw[window(j), k] / nd (gw_ldscore.py:2197, :2220-2222
-// applied per window).
+// Finalize of an estimate: meansq = sum of the probe slices (not written when
+// null) and ld = meansq / nvecs - Mkw[window(j), k] / nd (gw_ldscore.py:2197,
+// :2220-2222 applied per window; win_of null: one window).
 __global__ void win_finalize_kernel(const double* __restrict__ acc, int slices, int64_t MK, int K,
                                     double nvecs, double nd, const int32_t* __restrict__ win_of,
                                     const double* __restrict__ mkw, double* __restrict__ ld,
@@ -79,8 +79,8 @@ __global__ void win_finalize_kernel(const double* __restrict__ acc, int slices, 
     for (int q = 1; q < slices; ++q) s += acc[(int64_t)q * MK + t];
     const int64_t j = t / K;
     const int k = (int)(t - j * K);
-    meansq[t] = s;
-    ld[t] = s / nvecs - mkw[(int64_t)win_of[j] * K + k] / nd;
+    if (meansq) meansq[t] = s;
+    ld[t] = s / nvecs - mkw[(win_of ? (int64_t)win_of[j] * K : 0) + k] / nd;
 }
 
 void launch_win_finalize(const double* acc, int slices, int64_t M, int K, double nvecs, double nd,

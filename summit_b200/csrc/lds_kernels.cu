@@ -52,8 +52,8 @@ __global__ void repack_kernel(const uint8_t* __restrict__ src, int64_t src_bytes
 // All samples in order: a thread makes 16 bytes of a row (rows of the image are a
 // multiple of 32 bytes), from five aligned words shifted together (rows of the
 // source start at any byte) where those lie inside the source row, else byte by
-// byte.  Bound by memory: 20,000 samples, 4,870 SNPs (49 MB in and out): 154 ->
-// RPK us (one byte per thread).
+// byte.  Bound by memory and by the few waves of a chunk: 20,000 samples, 4,000
+// SNPs (40 MB in and out): 78 -> 15 us (one byte per thread).
 __global__ void repack_rows_kernel(const uint8_t* __restrict__ src, int64_t src_bytes, int64_t N,
                                    int64_t nbp, int64_t M, int64_t M_pad, uint8_t* __restrict__ dst) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
