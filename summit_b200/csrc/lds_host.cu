@@ -2067,6 +2067,8 @@ std::unique_ptr<GwPlan> plan_create(Context& c, std::shared_ptr<Prepared> P, con
         pl->ycs.as<double>((size_t)(K * vpmax));
     }
     pl->accum.as<double>((size_t)(M * K));
+    pl->ld_d.as<double>((size_t)(M * K));   // (here, so that the first results() allocates nothing)
+    pl->mk_d.as<double>((size_t)K);
     if (with_mc) pl->mc.as<double>((size_t)(M * K));
     pl->guards.as<unsigned long long>(2);
     ck(cudaStreamSynchronize(c.st), "plan");
