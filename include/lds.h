@@ -313,7 +313,7 @@ int lds_win_plan_bin_totals(int64_t plan, double* mkw_out);
  * knob; summit_b200/autotune.py chooses it, with the window batch size, by
  * timing):
  *   p1_sb_per_cta: phase-1 super-bins (window x bin) per CTA, i.e. how the
- *     super-bin work list is split across CTAs (0: default 8).
+ *     super-bin work list is split across CTAs (0: chosen from the launch's size).
  * The LD scores do not depend on the tiling (bit for bit).  No reference
  * counterpart (it replaces the reference's CPU tiling environment knobs). */
 int lds_win_plan_set_tiling(int64_t plan, int p1_sb_per_cta);

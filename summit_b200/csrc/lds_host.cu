@@ -1869,6 +1869,7 @@ struct GwPlan {
         Csr csr;
         DevBuf rowind, sc, binoff, wqoff, z, wq, wcs;
         int64_t lmax = 0;     // tcgen05 phase 1: padded member-list length
+        int p1_sb = 1;        // and super-bins per CTA
     };
     std::vector<std::unique_ptr<Tile>> tiles;
     DevBuf y, yq, ycs, accum, mc, lscale, guards, status;
@@ -2020,6 +2021,8 @@ std::unique_ptr<GwPlan> plan_create(Context& c, std::shared_ptr<Prepared> P, con
         if (tc) {
             for (int64_t kk = 0; kk < K; ++kk)
                 t->lmax = std::max(t->lmax, cs.bin_off[(size_t)kk + 1] - cs.bin_off[(size_t)kk]);
+            t->p1_sb = umma::choose_sb_per_cta(cs.bin_off.data(), (int)K, umma::ncolp_for(V),
+                                               P->g.N_pad / 128, (int)K);
             t->wq.as<int8_t>(std::max<size_t>(
                 umma::w_digit_bytes(cs.bin_off[(size_t)K], umma::ncolp_for(V)), 16));
             t->wcs.as<double>((size_t)(K * V));
@@ -2137,6 +2140,7 @@ void plan_enqueue_phase1(Context& c, GwPlan& pl, size_t ti, double* y, cudaEvent
         pa.status = static_cast<unsigned*>(pl.status.p);
         pa.m_pad = P.g.M_pad;
         pa.lmax = t.lmax;
+        pa.sb_per_cta = t.p1_sb;
         umma::launch_p1_umma(pa, P.g.N_pad, c.st);
     } else {
         launch_p1_weights(w, static_cast<double*>(P.d_mean.p), static_cast<double*>(P.d_sdinv.p),
@@ -2376,6 +2380,7 @@ struct WinPlan {
     std::vector<double> inv, Mkw;       // Mkw[w*K + k]
     struct Batch {
         int64_t w0 = 0, w1 = 0, ksup = 0, lmax = 0;
+        std::vector<int> p1_sb;            // phase-1 super-bins per CTA, per V-tile
         Csr csr;
         DevBuf rowind, sc, binoff, tiles;
         int64_t ntiles = 0;                // 128-SNP tiles
@@ -2597,6 +2602,9 @@ std::unique_ptr<WinPlan> win_plan_create(Context& c, std::shared_ptr<Prepared> P
             }
         }
         cs.bin_off[(size_t)b.ksup] = off;
+        for (int V : pl->vt)
+            b.p1_sb.push_back(umma::choose_sb_per_cta(cs.bin_off.data(), (int)b.ksup,
+                                                      umma::ncolp_for(V), Np / 128, (int)K));
         const size_t nm = std::max<size_t>(ri.size(), 1);
         h2d(b.rowind.as<int32_t>(nm), ri.data(), ri.size(), c.st);
         h2d(b.sc.as<double>(nm), scv.data(), scv.size(), c.st);
@@ -2757,9 +2765,9 @@ void win_enqueue(Context& c, WinPlan& pl) {
             static const int spc = [] {
                 const char* e = std::getenv("LDS_P1_SB_PER_CTA");
                 const int v = e ? std::atoi(e) : 0;
-                return v > 0 ? v : 8;
+                return v > 0 ? v : 0;
             }();
-            pa.sb_per_cta = pl.p1_spc > 0 ? pl.p1_spc : spc;
+            pa.sb_per_cta = pl.p1_spc > 0 ? pl.p1_spc : spc > 0 ? spc : b.p1_sb[ti];
             pa.yq = static_cast<int8_t*>(pl.yq->p);
             pa.ycolscale = static_cast<double*>(pl.ycs.p);
             pa.yshift = static_cast<int*>(pl.yshift.p);

@@ -154,6 +154,10 @@ struct P1UArgs {
     int64_t m_pad = 0;                  // image rows, for the bounds-checked build (0: unchecked)
 };
 
+// Super-bins per phase-1 CTA for the member lists off[0..K] (host memory) over
+// `tiles` sample tiles; `period` super-bins make a window (lds_umma_p1.cu).
+int choose_sb_per_cta(const int64_t* off, int K, int ncolp, int64_t tiles, int period);
+
 // Rows of a weight-digit tile in shared memory.
 __host__ __device__ inline int p1_tile_rows(const P1UArgs& a) {
     return a.share > 1 ? a.share * a.ncolp : (a.ncolp < 256 ? a.ncolp : 256);

@@ -131,6 +131,33 @@ def test_window_ld_pairs(oracle, n, m, K, reach, row0):
     sess.close()
 
 
+# The launch shapes chosen from a plan's sizes (several windows per phase-1 CTA
+# with a partial last group; bins shared out evenly among phase-2 CTAs) leave every
+# bit as one super-bin and one bin per CTA give it.
+@pytest.mark.parametrize("n,m,W,K,B", [(300, 1200, 9, 6, 10), (1500, 2600, 70, 5, 20), (140, 500, 2, 3, 50)])
+def test_launch_shapes(n, m, W, K, B):
+    from summit_b200.session import GwSession, WinPlan
+
+    rng = np.random.default_rng(m)
+    rows = _rows(n, m, seed=m)
+    annot = (rng.random((m, K)) < 0.3).astype(float)
+    annot[:, 0] = 1.0
+    cuts = np.sort(rng.choice(np.arange(1, m), W - 1, replace=False))
+    ws = np.concatenate([[0], cuts, [m]]).astype(np.int64)
+    sess = GwSession(rows, n)
+    out = []
+    for shape in (None, 1):
+        plan = WinPlan(sess, annot, ws, B, 250, 5)
+        if shape:
+            plan.set_tiling(shape)
+            plan.set_p2_bins(shape)
+        plan.execute()
+        out.append(plan.results()["ldscore"])
+        plan.close()
+    np.testing.assert_array_equal(out[0], out[1])
+    sess.close()
+
+
 # The per-block calls' sketch crosses PCIe in pieces of whole columns: 300,007
 # samples make a column longer than a piece, 60,001 ones several pieces of four
 # columns with a last partial one; a second block merges into the first's.
