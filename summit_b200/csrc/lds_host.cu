@@ -3300,6 +3300,7 @@ struct GxeCtx {
     // workspaces (grow-only)
     DevBuf probes, annot, sx, sw, panel, y, wq, wcs, rowind, sc, binoff, coef, coef2, denom, leak;
     DevBuf sacc, acc4, guards, status, flag;
+    DevBuf mrows, mcount;                // source members per annotation column
     DevBuf dgeno, dw, ones_L;            // dense-block path
     // Exact checks of the target's phase-2 products (lds_gxe_set_checks):
     // per-SNP checksums from the tensor-core epilogue (lhs) and from the
@@ -3356,11 +3357,34 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
     unsigned* flag = g.flag.as<unsigned>(1);
     ck(cudaMemsetAsync(flag, 0, 4, c.st), "memset");
     launch_gxe_check(dz, L * B, dsx, dsw, L * T, da, is_sqrt ? 0 : L * K, flag, c.st);
-    // Member lists need the annotation and scales on the host.
-    std::vector<double> ha((size_t)(L * K)), hx((size_t)(L * T)), hw((size_t)(L * T));
-    d2h(ha.data(), da, ha.size(), c.st);
-    d2h(hx.data(), dsx, hx.size(), c.st);
-    d2h(hw.data(), dsw, hw.size(), c.st);
+    const int nc = umma::ncolp_for((int)B);
+    // SNP chunks bound the weight-digit buffer (G x 2 x ncolp x chunk bytes).
+    const int64_t cap = (int64_t)1 << 30;
+    int64_t Lb = std::max<int64_t>(128, cap / std::max<int64_t>(1, G * 2 * nc) / 128 * 128);
+    Lb = std::min(Lb, round_up(L, 128));
+    // Members of each annotation column among SNPs [a, b) of the block (sqrt(a_jk) > 0),
+    // their numbers on the host once the stream has been waited for.
+    std::vector<int> members((size_t)K);
+    int32_t* drows = nullptr;
+    int* dcount = nullptr;
+    auto find_members = [&](int64_t a, int64_t b) {
+        drows = g.mrows.as<int32_t>((size_t)(K * Lb));
+        dcount = g.mcount.as<int>((size_t)K);
+        launch_gxe_members(da, L, a, b, (int)K, is_sqrt, Lb, drows, dcount, c.st);
+        d2h(members.data(), dcount, (size_t)K, c.st);
+    };
+    // (dense blocks form their weights from the annotation and scales on the host)
+    std::vector<double> ha, hx, hw;
+    if (dense) {
+        ha.resize((size_t)(L * K));
+        hx.resize((size_t)(L * T));
+        hw.resize((size_t)(L * T));
+        d2h(ha.data(), da, ha.size(), c.st);
+        d2h(hx.data(), dsx, hx.size(), c.st);
+        d2h(hw.data(), dsw, hw.size(), c.st);
+    } else {
+        find_members(0, std::min(L, Lb));
+    }
     unsigned fv = 0;
     d2h(&fv, flag, 1, c.st);
     ck(cudaStreamSynchronize(c.st), "gxe inputs");
@@ -3416,46 +3440,28 @@ void gxe_source_impl(Context& c, GxeCtx& g, int64_t j0, int64_t j1, const double
         return;
     }
     const Prepared& P = *g.P;
-    const int nc = umma::ncolp_for((int)B);
-    // SNP chunks bound the weight-digit buffer (G x 2 x ncolp x chunk bytes).
-    const int64_t cap = (int64_t)1 << 30;
-    int64_t Lb = std::max<int64_t>(128, cap / std::max<int64_t>(1, G * 2 * nc) / 128 * 128);
-    Lb = std::min(Lb, round_up(L, 128));
     double* Y = g.y.as<double>((size_t)(Np * C));
     for (int64_t a = 0; a < L; a += Lb) {
         const int64_t b = std::min(L, a + Lb), Lc = b - a;
-        // Super-bin (e, h, k): members with sqrt(a_jk) > 0, scale sqrt(a_jk) s_h,e[j].
+        if (a > 0) {
+            find_members(a, b);
+            ck(cudaStreamSynchronize(c.st), "gxe members");
+        }
+        // Super-bin (e, h, k): the members of bin k, scale sqrt(a_jk) s_h,e[j].
         std::vector<int64_t> off((size_t)G + 1, 0);
-        std::vector<int32_t> ri;
-        std::vector<double> scv;
         int64_t lmax = umma::kP1Step;
-        for (int64_t e = 0; e < T; ++e)
-            for (int h = 0; h < 2; ++h)
-                for (int64_t k = 0; k < K; ++k) {
-                    const int64_t gi = (e * 2 + h) * K + k;
-                    off[(size_t)gi] = (int64_t)ri.size();
-                    const double* s = (h == 0 ? hx.data() : hw.data()) + e * L;
-                    for (int64_t j = a; j < b; ++j) {
-                        const double av = ha[(size_t)(k * L + j)];
-                        const double sa = is_sqrt ? av : std::sqrt(std::max(0.0, av));
-                        if (!(sa > 0.0)) continue;
-                        ri.push_back((int32_t)(j - a));
-                        scv.push_back(sa * s[j]);
-                    }
-                    const int64_t n = (int64_t)ri.size() - off[(size_t)gi];
-                    const int64_t np = round_up(n, umma::kP1Step);
-                    for (int64_t q = n; q < np; ++q) {
-                        ri.push_back(0);
-                        scv.push_back(0.0);
-                    }
-                    lmax = std::max(lmax, np);
-                }
-        off[(size_t)G] = (int64_t)ri.size();
-        const size_t nm = std::max<size_t>(ri.size(), 1);
-        h2d(g.rowind.as<int32_t>(nm), ri.data(), ri.size(), c.st);
-        h2d(g.sc.as<double>(nm), scv.data(), scv.size(), c.st);
-        h2d(g.binoff.as<int64_t>(off.size()), off.data(), off.size(), c.st);
-        int8_t* wq = g.wq.as<int8_t>(std::max<size_t>(umma::w_digit_bytes((int64_t)ri.size(), nc), 16));
+        for (int64_t gi = 0; gi < G; ++gi) {
+            const int64_t np = round_up(members[(size_t)(gi % K)], umma::kP1Step);
+            off[(size_t)gi + 1] = off[(size_t)gi] + np;
+            lmax = std::max(lmax, np);
+        }
+        const int64_t listed = off[(size_t)G];
+        const size_t nm = (size_t)std::max<int64_t>(listed, 1);
+        int64_t* doff = g.binoff.as<int64_t>(off.size());
+        h2d(doff, off.data(), off.size(), c.st);
+        launch_gxe_lists(da, dsx, dsw, L, a, (int)K, G, is_sqrt, Lb, drows, dcount, doff,
+                         listed > 0 ? lmax : 0, g.rowind.as<int32_t>(nm), g.sc.as<double>(nm), c.st);
+        int8_t* wq = g.wq.as<int8_t>(std::max<size_t>(umma::w_digit_bytes(listed, nc), 16));
         umma::P1UWeights uw;
         uw.K = (int)G;
         uw.V = (int)B;

@@ -159,6 +159,12 @@ void launch_gxe_target_finalize(const double* S, int64_t L, int Kp, int K, int T
                                 int env_start, int64_t total, int64_t block_start, double* a0,
                                 double* a1, double* a2, double* a3, cudaStream_t st);
 void launch_scale(double* x, int64_t n, double s, cudaStream_t st);
+void launch_gxe_members(const double* annot, int64_t L, int64_t a, int64_t b, int K, int is_sqrt,
+                        int64_t cap, int32_t* rows, int* count, cudaStream_t st);
+void launch_gxe_lists(const double* annot, const double* sx, const double* sw, int64_t L, int64_t a,
+                      int K, int64_t G, int is_sqrt, int64_t cap, const int32_t* rows,
+                      const int* count, const int64_t* off, int64_t longest, int32_t* rowind,
+                      double* sc, cudaStream_t st);
 void launch_gxe_check(const double* probes, int64_t np, const double* sx, const double* sw,
                       int64_t ns, const double* annot, int64_t na, unsigned* flag, cudaStream_t st);
 void launch_philox_rademacher(const uint64_t* keys, int64_t P, int64_t rows, double* out,

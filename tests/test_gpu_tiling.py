@@ -158,6 +158,43 @@ def test_launch_shapes(n, m, W, K, B):
     sess.close()
 
 
+# GxE source member lists made on the device: several columns of different density
+# (one empty), more than one pass of 1,024 SNPs, a list of exactly one K-step, both
+# annotation forms, against the same products of a dense standardized block, whose
+# weights the host forms.
+@pytest.mark.parametrize("m,start,K,is_sqrt", [(2500, 0, 3, False), (1100, 13, 4, True), (64, 0, 1, False)])
+def test_gxe_member_lists(m, start, K, is_sqrt):
+    from oracle.gxe_oracle import design
+    from summit_b200 import bedfile, gxeldcore
+    from summit_b200.session import GwSession
+
+    n, T, B = 260, 2, 5
+    rng = np.random.default_rng(m + K)
+    g = rng.binomial(2, 0.3, (m, n)).astype(np.int8)
+    g[rng.random((m, n)) < 0.02] = -9
+    sess = GwSession(bedfile.pack_bed_rows(g), n)
+    mean, sdinv = (sess.stats()[key] for key in ("mean", "sdinv"))
+    X = np.where(g < 0, 0.0, (g - mean[:, None]) * sdinv[:, None]).T
+    d = design(n, T, seed=1)
+    k = gxeldcore.MultiEnvironmentKernel(d["environments"], d["feature_basis"],
+                                         d["power_indices"], d["power_offsets"], d["ranks"],
+                                         d["gram_values"], d["gram_offsets"], d["e2_gram_values"],
+                                         d["common_basis"], d["directions"], 1, K, 2)
+    L = m - start
+    ann = rng.random((L, K)) * (rng.random((L, K)) < np.linspace(1.0, 0.05, K))
+    if K > 1:
+        ann[:, 1] = 0.0
+    z = rng.choice([-1.0, 1.0], (L, B))
+    sx, sw = rng.random((L, T)) + 0.5, rng.random((L, T)) + 0.5
+    out = []
+    for block in (sess.block(start, m), np.asfortranarray(X[:, start:])):
+        target = np.zeros((n, T * 2 * K * B), order="F")
+        assert k.source_block(target, block, z, ann, sx, sw, 0, annotation_is_sqrt=is_sqrt) == 0
+        out.append(target)
+    assert rel_err(out[0], out[1]) < TOL
+    sess.close()
+
+
 # The per-block calls' sketch crosses PCIe in pieces of whole columns: 300,007
 # samples make a column longer than a piece, 60,001 ones several pieces of four
 # columns with a last partial one; a second block merges into the first's.
