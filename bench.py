@@ -150,6 +150,13 @@ def reference_sample(m_sample: int, tmpdir: str, packed=None) -> tuple[str, np.n
     return prefix, annotations(M_SNPS)[:m_sample]
 
 
+def reference_built() -> bool:
+    """Whether the reference's own gwldcore.cpp has been compiled here (oracle/_ref)."""
+    from oracle.oracle import REF_SO
+
+    return REF_SO.exists()
+
+
 def run_reference_windows(packed: np.ndarray, annot: np.ndarray, ws: np.ndarray, threads: int,
                           tmpdir: str) -> float:
     """The reference's per-block native calls run window by window (each window
@@ -691,7 +698,10 @@ def ours_arm(args) -> None:
             line["product_checks"] = product_checks
         if lvp is not None:
             line["learned_vs_plain"] = lvp
-        if world == 1 and not os.environ.get("LDS_SKIP_CPU_BASELINE"):
+        if world == 1 and not reference_built():
+            line["cpu_baseline"] = {"unavailable": "the reference's CPU library is not built "
+                                                   "(make -C oracle ref needs its sources)"}
+        elif world == 1 and not os.environ.get("LDS_SKIP_CPU_BASELINE"):
             threads = cpu_threads()
             with tempfile.TemporaryDirectory() as td:
                 pk, ann_s, ws_s = reference_sample_windows(
