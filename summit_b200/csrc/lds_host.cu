@@ -98,20 +98,30 @@ struct PoolScope {
     ~PoolScope() { t_pool = saved; }
 };
 
-// The pool of buffers that live for one call (CallScope); null until first used.
+// The pool of buffers that live for one call (CallScope), null until first used,
+// and the bytes that it has handed out (both change under the context's lock).
+// Buffers above kCallPoolBuf, and any that would take it above kCallPoolKeep, are
+// ordinary memory: the pool maps new memory at 6 to 70 ms per GB and unmaps what it
+// may not keep at as much, where cudaMalloc takes under 1 ms (a GxE right pair of
+// 2.6 GB: 728 ms).
 cudaMemPool_t g_call_pool = nullptr;
+size_t g_call_pool_live = 0;
+constexpr size_t kCallPoolBuf = 128ull << 20;
+constexpr size_t kCallPoolKeep = 512ull << 20;
 
 struct DevBuf {
     void* p = nullptr;
     size_t n = 0;
     cudaStream_t pool_st = nullptr;  // non-null: pool memory, freed in this stream's order
+    bool call_mem = false;           // and of the call pool
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), pool_st(o.pool_st) {
+    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n), pool_st(o.pool_st), call_mem(o.call_mem) {
         o.p = nullptr;
         o.n = 0;
         o.pool_st = nullptr;
+        o.call_mem = false;
     }
     DevBuf& operator=(DevBuf&& o) noexcept {
         if (this != &o) {
@@ -119,9 +129,11 @@ struct DevBuf {
             p = o.p;
             n = o.n;
             pool_st = o.pool_st;
+            call_mem = o.call_mem;
             o.p = nullptr;
             o.n = 0;
             o.pool_st = nullptr;
+            o.call_mem = false;
         }
         return *this;
     }
@@ -129,9 +141,13 @@ struct DevBuf {
         if (bytes <= n && p) return p;
         release();
         if (bytes == 0) bytes = 16;
-        if (t_pool.pool) {
+        const bool call = t_pool.pool && t_pool.pool == g_call_pool;
+        if (t_pool.pool && !(call && (bytes > kCallPoolBuf ||
+                                      g_call_pool_live + bytes > kCallPoolKeep))) {
             ck(cudaMallocFromPoolAsync(&p, bytes, t_pool.pool, t_pool.st), "pool allocation");
             pool_st = t_pool.st;
+            call_mem = call;
+            if (call) g_call_pool_live += bytes;
         } else {
             cudaError_t e = cudaMalloc(&p, bytes);
             if (e == cudaErrorMemoryAllocation && g_call_pool) {  // give back what it holds unused
@@ -149,12 +165,14 @@ struct DevBuf {
     T* as(size_t count) { return static_cast<T*>(get(count * sizeof(T))); }
     void release() {
         if (p) {
+            if (call_mem) g_call_pool_live -= n;
             if (pool_st) cudaFreeAsync(p, pool_st);
             else cudaFree(p);
         }
         p = nullptr;
         n = 0;
         pool_st = nullptr;
+        call_mem = false;
     }
     ~DevBuf() { release(); }
 };
@@ -310,7 +328,6 @@ void ensure_device(Context& c) {
 // kCallPoolKeep unused across calls; lds_clear_device_cache and a failing
 // allocation give that back too.  The scope ends with the stream idle, so that a
 // call that failed leaves no copy from the caller's memory in flight.
-constexpr uint64_t kCallPoolKeep = 512ull << 20;
 
 cudaMemPool_t call_pool(Context& c) {
     if (!g_call_pool) {
