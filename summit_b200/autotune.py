@@ -7,7 +7,7 @@ device work of a windowed estimate are chosen by timing them on the device:
 
 * ``p1_sb_per_cta``: how the phase-1 work list of (window, bin) super-bins is
   split across CTAs (super-bins per CTA: longer per-CTA pipelines against
-  more CTAs to balance);
+  more CTAs to balance; 0: chosen from the lists' lengths);
 * ``batch_gb``: how the windows are split into launches (the sketch digits of
   one batch stay under this many GB);
 * ``p2_bin_chunk``: the phase-2 CTA order (window by window, chunks of about
@@ -36,7 +36,7 @@ from typing import Callable, Iterable
 
 import numpy as np
 
-DEFAULT_CONFIG = {"p1_sb_per_cta": 8, "batch_gb": 8.0, "p2_bin_chunk": 4, "p2_bins": 0}
+DEFAULT_CONFIG = {"p1_sb_per_cta": 0, "batch_gb": 8.0, "p2_bin_chunk": 4, "p2_bins": 0}
 
 
 def default_candidates() -> list[dict]:
