@@ -5,6 +5,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "lds_p1_shape.h"
+
 namespace lds {
 namespace umma {
 
@@ -110,9 +112,6 @@ inline int p2_bins_per_cta_grouped(int ncolp, int K) {
     return best;
 }
 
-// Member SNPs per phase-1 K-step: member lists are padded to a multiple of it.
-constexpr int kP1Step = 64;
-
 // Phase-1 weight digits, column col of part 0 (W1) or 1 (-W2) for member r of
 // K-step `step` (counted over all super-bins' lists): a step's columns are
 // contiguous 128-byte rows, the step's members of W1 and then of -W2,
@@ -153,10 +152,6 @@ struct P1UArgs {
     const int* yshift = nullptr;        // K*V digit shifts eW - eY (from the weight kernel)
     int64_t m_pad = 0;                  // image rows, for the bounds-checked build (0: unchecked)
 };
-
-// Super-bins per phase-1 CTA for the member lists off[0..K] (host memory) over
-// `tiles` sample tiles; `period` super-bins make a window (lds_umma_p1.cu).
-int choose_sb_per_cta(const int64_t* off, int K, int ncolp, int64_t tiles, int period);
 
 // Rows of a weight-digit tile in shared memory.
 __host__ __device__ inline int p1_tile_rows(const P1UArgs& a) {

@@ -33,7 +33,6 @@
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
-#include <map>
 
 #include "lds_internal.h"
 #include "lds_tc.cuh"
@@ -720,52 +719,6 @@ size_t p1_umma_smem_bytes(int tile_rows) { return (size_t)p1::Layout(tile_rows).
 void prepare_p1_umma() {
     cudaFuncSetAttribute(p1_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          p1::kSmemLimit);
-}
-
-// The number with the earliest estimated end of the launch.  A CTA pays about
-// 10,000 cycles before its pipeline runs, then per super-bin the epilogue's
-// share and its K-steps (fits of measured launches); tiles CTAs of each group go
-// to the SMs in launch order.  Beyond 12 waves the sum and half the longest CTA
-// stand for that walk.  More per CTA than needed leave a long last wave and mix
-// long lists with short ones; hence whole windows or even parts of one, up to 64.
-// Windowed, 8 per CTA -> this choice: N = 50,000, M = 60,000, K = 24, B = 50:
-// 8.1 -> 7.2 ms; N = 10,007, K = 6, B = 10: 113 -> 104 us; genome-wide, 1 per CTA ->
-// this choice: N = 50,000, M = 40,000, K = 24, B = 50: 1.95 -> 1.75 ms.
-int choose_sb_per_cta(const int64_t* off, int K, int ncolp, int64_t tiles, int period) {
-    constexpr double kSms = 148.0, kStart = 10000.0;
-    const double per_job = 2000.0 * ((ncolp + 255) / 256);
-    const double per_member = (200.0 + 1.5 * ncolp) / kP1Step;
-    int best = 1;
-    double least = 0.0;
-    for (int s = 1; s <= std::min(K, 64); ++s) {
-        if (s % period != 0 && period % s != 0) continue;
-        const int groups = (K + s - 1) / s;
-        const bool walk = (double)tiles * groups <= 12.0 * kSms;
-        std::map<double, int64_t> free_at;   // when how many SMs are free
-        free_at[0.0] = (int64_t)kSms;
-        double sum = 0.0, longest = 0.0, end = 0.0;
-        for (int g = 0; g < groups; ++g) {
-            const int q0 = g * s, q1 = std::min(K, q0 + s);
-            const double c = kStart + (q1 - q0) * per_job + (double)(off[q1] - off[q0]) * per_member;
-            sum += c;
-            longest = std::max(longest, c);
-            for (int64_t left = walk ? tiles : 0; left > 0;) {
-                const auto first = free_at.begin();
-                const int64_t n = std::min(left, first->second);
-                const double done = first->first + c;
-                if ((first->second -= n) == 0) free_at.erase(first);
-                free_at[done] += n;
-                end = std::max(end, done);
-                left -= n;
-            }
-        }
-        if (!walk) end = sum * (double)tiles / kSms + 0.5 * longest;
-        if (s == 1 || end < least) {
-            least = end;
-            best = s;
-        }
-    }
-    return best;
 }
 
 void launch_p1_umma(const P1UArgs& a, int64_t N_pad, cudaStream_t st) {

@@ -1,0 +1,58 @@
+"""Phase-1 host logic, compiled from the library's own headers with the host
+compiler (no CUDA): the launch shape."""
+from __future__ import annotations
+
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+def run_cpp(tmp_path, body: str, *flags: str) -> str:
+    """Compile `body` against summit_b200/csrc and run it."""
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(body)
+    subprocess.run(["g++", "-std=c++17", "-O1", *flags, "-I", str(ROOT / "summit_b200" / "csrc"),
+                    str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+
+
+SHAPE = """
+#include <cstdio>
+#include <vector>
+#include "lds_p1_shape.h"
+int main() {
+    const int K = %d, W = %d, members = %d;
+    std::vector<int64_t> off{0};
+    for (int q = 0; q < K * W; ++q) off.push_back(off.back() + members);
+    std::printf("%%d", lds::umma::choose_sb_per_cta(off.data(), K * W, %d, %d, K));
+}
+"""
+
+
+# Windowed plans took 8 super-bins per CTA before the choice: a number of bins
+# with no divisor near 8 is not left with 1, whose CTAs are mostly start-up.
+@pytest.mark.parametrize("K", [67, 97, 134])
+@pytest.mark.parametrize("W,tiles", [(20, 40), (700, 391)])
+def test_bins_with_few_divisors_share_a_cta(tmp_path, K, W, tiles):
+    assert int(run_cpp(tmp_path, SHAPE % (K, W, 128, 208, tiles))) >= 8
+
+
+# The super-bins' CTAs lie along grid.y, which holds 65,535: 97 bins x 700 windows
+# at one per CTA would not fit, nor 24 x 3,000 (or x 200,000) at few per CTA.
+@pytest.mark.parametrize("K,W", [(97, 700), (24, 3000), (1, 70000), (24, 200000)])
+def test_the_grid_holds_the_ctas(tmp_path, K, W):
+    s = int(run_cpp(tmp_path, SHAPE % (K, W, 64, 48, 2)))
+    assert 1 <= s <= 256 and -(-K * W // s) <= 65535
+
+
+# 8 windows x 23 bins over 40 sample tiles: whole windows are estimated 2.6 %
+# earlier than 8 per CTA, within the estimate's own error.
+def test_a_near_tie_keeps_the_plain_number(tmp_path):
+    assert int(run_cpp(tmp_path, SHAPE % (23, 8, 128, 80, 40))) == 8
+
+
+def test_even_parts_of_a_window(tmp_path):
+    assert int(run_cpp(tmp_path, SHAPE % (24, 60, 128, 208, 391))) in (8, 12, 24, 48)
