@@ -6,6 +6,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "lds_digits.h"
+
 #include "lds_device.cuh"
 #include "lds_internal.h"
 
@@ -232,18 +234,6 @@ __device__ __forceinline__ void decode_row_sw128(uint4 p0, uint4 p1, uint8_t* gR
         *reinterpret_cast<uint4*>(gRow + off) = make_uint4(g0, g1, g2, g3);
         *reinterpret_cast<uint4*>(oRow + off) = make_uint4(o0, o1, o2, o3);
     }
-}
-
-// The balanced base-128 digits of a 28-bit sketch value R = d0 128^3 + d1 128^2
-// + d2 128 + d3 (d1..d3 in [-63, 64]) as the bytes of one word, d3 lowest.
-// U = R + 63 (128^2 + 128 + 1) has the digits' 7-bit fields (plus 63) in place;
-// two multiply-adds spread them to bytes (top field first by 2, then the upper
-// field of each half by 1), and adding 65 and flipping the top bit subtracts 63
-// from each of the low three bytes without a borrow.
-__device__ __forceinline__ uint32_t digits_word(int R) {
-    const uint32_t U = (uint32_t)(R + 63 * (16384 + 128 + 1));
-    const uint32_t y = U + 3u * (U & 0xFFFFC000u);
-    return (y + (y & 0xFF803F80u) + 0x00414141u) ^ 0x00808080u;
 }
 
 // Index checks of the bounds-checked build (-DLDS_CHECKED): a failed check

@@ -398,9 +398,8 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     const int v = g * 64 + 8 * (h + 2 * (lane >> 3)) + (lane & 7);
                     const int r = v < a.V ? -a.yshift[(int64_t)k * a.V + v] : 0;
                     narrow = small_sums && __all_sync(0xffffffffu, r >= 0 && r <= 14);
-                    // x = right shift, y = 14 - x, z = half an ulp less one, w = parity mask
-                    tab[lane] = make_int4(r, 14 - r, r > 0 ? (1 << ((r - 1) & 15)) - 1 : 0,
-                                          r > 0 ? 1 : 0);
+                    const NarrowShift sh = narrow_shift(r);
+                    tab[lane] = make_int4(sh.r, sh.up, sh.half, sh.odd);
                     __syncwarp();
                 } else {
                     const int64_t oa = probe_of(g * 64 + lane, nbin), ob = probe_of(g * 64 + lane + 32, nbin);
@@ -429,11 +428,8 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
                     // s / 16 = 2q + a / 4, swizzled with the row's low three bits,
                     // (4 v + t) & 7 = 4 (v & 1) + t.
                     //
-                    // R in 32 bits (`narrow`): T = H 2^14 + L with H = 128 t0 + t1 and
-                    // L = 128 t2 + t3 (|L| < 2^31 up to kMaxNarrowSteps K-steps), so for
-                    // 0 <= r <= 14 R = H 2^(14-r) + rint(L 2^-r), the tie parity taken
-                    // from the whole value; H's multiple may wrap, R does not.  19
-                    // instructions per (sample, probe) instead of the 64-bit form's ~60.
+                    // R in 32 bits (`narrow`) where 0 <= r <= 14 and the low digits' part
+                    // stays below 2^31 (up to kMaxNarrowSteps K-steps): narrow_round.
                     const int qd = lane & 3;
                     // word byte b holds digit 3 - b: lane t of a quad keeps byte 3 - t
                     const uint32_t selA = qd < 2 ? 0x7632u : 0x1054u;
@@ -457,11 +453,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
 #pragma unroll
                             for (int p = 0; p < 8; ++p) {
                                 const int4 sh = tab[cc + p];
-                                const int L = rr[4 * p + 2] * 128 + rr[4 * p + 3];
-                                const int A = (int)((uint32_t)(rr[4 * p] * 128 + rr[4 * p + 1])
-                                                    << sh.y);
-                                const int odd = (A + (L >> sh.x)) & sh.w;
-                                R[p] = A + ((L + sh.z + odd) >> sh.x);
+                                R[p] = narrow_round(rr[4 * p], rr[4 * p + 1], rr[4 * p + 2],
+                                                    rr[4 * p + 3],
+                                                    NarrowShift{sh.x, sh.y, sh.z, sh.w});
                             }
                         } else {
 #pragma unroll

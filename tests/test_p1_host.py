@@ -56,3 +56,52 @@ def test_a_near_tie_keeps_the_plain_number(tmp_path):
 
 def test_even_parts_of_a_window(tmp_path):
     assert int(run_cpp(tmp_path, SHAPE % (24, 60, 128, 208, 391))) in (8, 12, 24, 48)
+
+
+DIGITS = """
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include "lds_digits.h"
+using namespace lds::umma;
+typedef long long ll;
+static uint64_t state = 7;
+static uint64_t rnd() {
+    state ^= state << 13, state ^= state >> 7, state ^= state << 17;
+    return state * 2685821657736338717ull;
+}
+static void check(int32_t t0, int32_t t1, int32_t t2, int32_t t3, int r) {
+    const ll T = (((ll)t0 * 128 + t1) * 128 + t2) * 128 + t3;
+    ll want = T >> r;                                    // to the nearest, ties to even
+    const ll rest = T - want * (1ll << r), half = r ? 1ll << (r - 1) : 1;
+    if (r && (rest > half || (rest == half && (want & 1)))) ++want;
+    if (std::llabs(want) > 127ll << 21) return;          // (the columns' scale: top digit at most 127)
+    const int32_t got = narrow_round(t0, t1, t2, t3, narrow_shift(r));
+    if (got != want) { std::printf("%d %d %d %d >> %d: %d, not %lld", t0, t1, t2, t3, r, got, want); std::exit(0); }
+    const uint32_t w = digits_word(got);
+    const ll back = (((ll)(int8_t)(w >> 24) * 128 + (int8_t)(w >> 16)) * 128 + (int8_t)(w >> 8)) * 128 + (int8_t)w;
+    if (back != got) { std::printf("digits of %d: %lld", got, back); std::exit(0); }
+}
+int main() {
+    const int32_t big = 85952 * 3 * 64;                  // digit products of the longest narrow list
+    for (int r = 0; r <= 14; ++r)
+        for (int n = 0; n < 200000; ++n) {
+            // a result R and low digits in range, and the high digits that go with them
+            const int32_t t2 = n % 3 ? (int32_t)(rnd() % (2u * big + 1)) - big : (n % 2 ? big : -big);
+            const int32_t t3 = n % 5 ? (int32_t)(rnd() % (2u * big + 1)) - big : (n % 2 ? big : -big);
+            const ll R = (ll)(rnd() % (1u << 29)) - (1 << 28);
+            const ll H = (R * (1ll << r) - ((ll)t2 * 128 + t3)) >> 14;
+            const int32_t t1 = (int32_t)(rnd() % 257) - 128;
+            check((int32_t)((H - t1) >> 7), (int32_t)(H - ((H - t1) >> 7) * 128), t2, t3, r);
+        }
+    digits_word(INT32_MAX), digits_word(INT32_MIN);      // (columns that are not finite)
+    std::printf("ok");
+}
+"""
+
+
+# The 32-bit rounding of the digit sums against 64-bit arithmetic, over low parts
+# up to the longest list's, where its terms wrap; no step of it may be undefined.
+def test_narrow_rounding(tmp_path):
+    assert run_cpp(tmp_path, DIGITS, "-fsanitize=undefined",
+                   "-fno-sanitize-recover=all") == "ok"
