@@ -35,6 +35,7 @@
 #include <cstdio>
 
 #include "lds_internal.h"
+#include "lds_p1_drain.h"
 #include "lds_tc.cuh"
 #include "lds_umma.h"
 
@@ -88,7 +89,21 @@ struct Layout {
 };
 static_assert(4 * (2 * kATile + 2 * 256 * kBK) + Layout::tail() + 1024 <= kSmemLimit,
               "four stages of 256 digit columns fit");
-static_assert((2 * kMaxStages + 5) * 8 + 8 <= 256, "the barriers fit");
+constexpr int kDecWarps = kSetWarps * kDecSets;
+static_assert((2 * kMaxStages + 5) * 8 + 8 + kDecWarps * 4 <= 256,
+              "the barriers, the abort flag and the decoders' positions fit");
+
+// (out of line: it is for the error path only)
+__device__ __noinline__ void settle(uint64_t* full, const volatile int* dec_next, int issued,
+                                    int nst) {
+    for (int w = 0; w < kDecWarps; ++w)
+        for (long long i = 0; dec_next[w] < 0 && i < wait_limit(); ++i) {
+        }
+    __threadfence_block();
+    p1_settle(issued, nst, kDecSets, kSetWarps,
+              [&](int w) { return dec_next[w] < 0 ? INT_MAX : dec_next[w]; },
+              [&](int st) { mbar_arrive(&full[st]); });
+}
 }  // namespace p1
 
 __global__ void __launch_bounds__(p1::kThreads, 1)
@@ -107,6 +122,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
     uint64_t* mma_done = acc_empty + 2;         // drain of the issuer's MMAs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* dec_next = abort_flag + 1;    // [kDecWarps] first step not arrived for, once left
     int4* shift_tab = reinterpret_cast<int4*>(smem + lay.shift_off());
     int* ktab = reinterpret_cast<int*>(smem + lay.table_off());
 
@@ -132,6 +148,7 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
         }
         mbar_init(mma_done, 1);
         *abort_flag = 0;
+        for (int w = 0; w < kDecWarps; ++w) dec_next[w] = -1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -185,8 +202,16 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             }
             // Drain: no tile copy may still be landing when the CTA exits
             // (only reachable with copies outstanding after an abort).
-            for (int j = max(0, it - nst); j < it; ++j)
-                mbar_wait(&full[j % nst], (uint32_t)(j / nst) & 1u);
+            bool settled = false;
+            for (int j = max(0, it - nst); j < it; ++j) {
+                const uint32_t par = (uint32_t)(j / nst) & 1u;
+                if (mbar_wait(&full[j % nst], par, abort_flag)) continue;
+                if (!settled) {
+                    settle(full, dec_next, it, nst);
+                    settled = true;
+                }
+                mbar_wait(&full[j % nst], par);
+            }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -332,6 +357,9 @@ __global__ void __launch_bounds__(p1::kThreads, 1)
             }
         }
         cp_async_wait_all();  // no gather copy may outlive the CTA (abort path)
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) dec_next[warp - kDecWarp0] = it;
     } else {
         // ---------------- epilogue (eight warps per accumulator) ----------------
         // Each half of the warps answers for one accumulator, so that the waits,

@@ -1,5 +1,6 @@
 """Phase-1 host logic, compiled from the library's own headers with the host
-compiler (no CUDA): the launch shape."""
+compiler (no CUDA): the launch shape, the
+digits' rounding, the drain after an abort."""
 from __future__ import annotations
 
 import subprocess
@@ -105,3 +106,44 @@ int main() {
 def test_narrow_rounding(tmp_path):
     assert run_cpp(tmp_path, DIGITS, "-fsanitize=undefined",
                    "-fno-sanitize-recover=all") == "ok"
+
+
+DRAIN = """
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+#include "lds_p1_drain.h"
+int main() {
+    srand(5);
+    const int sets = 4, warps = 2;
+    for (int n = 0; n < 20000; ++n) {
+        // Steps [0, used) consumed, [0, issued) issued by the producer, each decoder
+        // warp stopped somewhere in the steps whose stages were free.
+        const int nst = 4 + rand() % 5, used = rand() % 40, issued = used + rand() % (nst + 1);
+        std::vector<int> next(sets * warps);
+        for (int w = 0; w < sets * warps; ++w) next[w] = used + rand() % (nst + 1);
+        // arrivals per step: the producer's and the warps'; steps share nst barriers
+        std::vector<int> got(issued + 2 * nst, 0);
+        for (int j = 0; j < issued + nst; ++j) {
+            if (j < issued) ++got[j];
+            for (int u = 0; u < warps; ++u)
+                if (next[(j % sets) * warps + u] > j) ++got[j];
+        }
+        lds::umma::p1_settle(issued, nst, sets, warps, [&](int w) { return next[w]; }, [&](int s) {
+            int j = issued - 1;              // the stage's step that is under way
+            while (j % nst != s) --j;
+            ++got[j];
+        });
+        for (int j = issued > nst ? issued - nst : 0; j < issued; ++j) {
+            if (got[j] != warps + 1) { std::printf("step %d of %d: %d arrivals", j, issued, got[j]); return 0; }
+        }
+    }
+    std::printf("ok");
+}
+"""
+
+
+# After an abort every stage that holds a copy in flight gets the arrivals its
+# barrier still needs, and no more, wherever the decoders stopped.
+def test_drain_completes_every_stage(tmp_path):
+    assert run_cpp(tmp_path, DRAIN) == "ok"
