@@ -150,11 +150,7 @@ struct Context {
     cudaMemPool_t pool = nullptr;   // chunk images and plans (PoolScope on st_prep)
     void* pinned = nullptr;
     size_t pinned_n = 0;
-    // Two pinned halves through which the per-block calls' sketches cross PCIe
-    // (kStageBytes each, or one column where that is longer), and their events.
-    void* stage = nullptr;
-    size_t stage_n = 0;
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    PinnedStage stage;   // through which the per-block calls' sketches cross PCIe
     KeptBuf y, yq, ycs, wq, wcs, z, rowind, sc, binoff, wqoff, accum, mc, guards, lscale, xin;
     KeptBuf colsum;  // per-block phase 2: sketch digit column sums (images with complete tiles)
     // Surrogate-network workspace, grow-only so that repeated training and
@@ -224,81 +220,6 @@ struct CallScope {
     explicit CallScope(Context& c) : st(c.st), scope(call_pool(c), c.st) {}
     ~CallScope() { cudaStreamSynchronize(st); }
 };
-
-// ---------------------------------------------------------------------------
-// Columns of doubles between a device array (ld >= rows) and host code that
-// converts or merges them, in pieces of whole columns through pinned memory, so
-// that one piece crosses PCIe while the host works on the other.  The per-block
-// calls (5,000 samples, 4,000 SNPs, K = 2, B = 20: 8 calls of 1.6 MB) moved a
-// column per copy through pageable memory: 8.2 -> 5.1 ms in all.
-// ---------------------------------------------------------------------------
-constexpr size_t kStageBytes = 2ull << 20;
-
-double* stage_half(Context& c, int h, int64_t rows, int64_t* cols_per_piece) {
-    const size_t col = sizeof(double) * (size_t)std::max<int64_t>(rows, 1);
-    const size_t half = std::max(kStageBytes, col);
-    for (cudaEvent_t& e : c.stage_ev)
-        if (!e) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-    if (c.stage_n < 2 * half) {
-        ck(cudaStreamSynchronize(c.st), "staging");
-        if (c.stage) cudaFreeHost(c.stage);
-        c.stage = nullptr;
-        c.stage_n = 0;
-        ck(cudaHostAlloc(&c.stage, 2 * half, cudaHostAllocDefault), "pinned staging");
-        c.stage_n = 2 * half;
-    }
-    *cols_per_piece = std::max<int64_t>(1, (int64_t)(half / col));
-    return reinterpret_cast<double*>(static_cast<char*>(c.stage) + (size_t)h * (c.stage_n / 2));
-}
-
-// use(q0, n, p): columns [q0, q0 + n) at p, `rows` apart, in order.
-template <typename F>
-void download_cols(Context& c, const double* d, int64_t ld, int64_t rows, int64_t cols, F&& use) {
-    int64_t per = 1;
-    stage_half(c, 0, rows, &per);
-    const int64_t pieces = (cols + per - 1) / per;
-    auto fetch = [&](int64_t i) {
-        const int64_t q0 = i * per, n = std::min(per, cols - q0);
-        ck(cudaMemcpy2DAsync(stage_half(c, (int)(i & 1), rows, &per), sizeof(double) * (size_t)rows,
-                             d + q0 * ld, sizeof(double) * (size_t)ld,
-                             sizeof(double) * (size_t)rows, (size_t)n, cudaMemcpyDeviceToHost, c.st),
-           "D2H");
-        ck(cudaEventRecord(c.stage_ev[i & 1], c.st), "event");
-    };
-    for (int64_t i = 0; i < std::min<int64_t>(2, pieces); ++i) fetch(i);
-    for (int64_t i = 0; i < pieces; ++i) {
-        ck(cudaEventSynchronize(c.stage_ev[i & 1]), "download");
-        const int64_t q0 = i * per;
-        use(q0, std::min(per, cols - q0),
-            static_cast<const double*>(stage_half(c, (int)(i & 1), rows, &per)));
-        if (i + 2 < pieces) fetch(i + 2);
-    }
-}
-
-// Columns h (T, `rows` apart) to d as FP64, rows..ld of each column zero.
-template <typename T>
-void upload_cols(Context& c, double* d, int64_t ld, const T* h, int64_t rows, int64_t cols) {
-    if (cols <= 0) return;
-    if (ld > rows)
-        ck(cudaMemset2DAsync(d + rows, sizeof(double) * (size_t)ld, 0,
-                             sizeof(double) * (size_t)(ld - rows), (size_t)cols, c.st),
-           "memset");
-    int64_t per = 1;
-    stage_half(c, 0, rows, &per);
-    ck(cudaStreamSynchronize(c.st), "staging");   // an earlier call's copies from the halves
-    const int64_t pieces = (cols + per - 1) / per;
-    for (int64_t i = 0; i < pieces; ++i) {
-        const int64_t q0 = i * per, n = std::min(per, cols - q0);
-        double* p = stage_half(c, (int)(i & 1), rows, &per);
-        if (i >= 2) ck(cudaEventSynchronize(c.stage_ev[i & 1]), "upload");
-        for (int64_t x = 0; x < n * rows; ++x) p[x] = (double)h[q0 * rows + x];
-        ck(cudaMemcpy2DAsync(d + q0 * ld, sizeof(double) * (size_t)ld, p,
-                             sizeof(double) * (size_t)rows, sizeof(double) * (size_t)rows, (size_t)n,
-                             cudaMemcpyHostToDevice, c.st),
-           "H2D");
-        ck(cudaEventRecord(c.stage_ev[i & 1], c.st), "event");
-    }
-}
 
 // Mean and inverse sd over observed calls (genotype.cpp:651-689).
 void stats_observed(long long nobs, long long sum, long long sumsq, int ddof, double& mu,
@@ -1602,27 +1523,8 @@ void phase1_bed_impl(const char* bed_prefix, const char* fam_path, int blk_start
         DevBuf tmp;
         project_cols(c, static_cast<double*>(c.y.p), P.g.N_pad, K * v_count, cv, false, tmp);
     }
-    // Download the block's contribution and merge with beta semantics.
-    std::vector<char> touched((size_t)K, 0), beta1((size_t)K, 1);
-    for (int64_t k = 0; k < K; ++k) {
-        if (csr.nnz[(size_t)k] == 0) continue;
-        touched[(size_t)k] = 1;
-        if (bin_init) beta1[(size_t)k] = bin_init[k] != 0;
-    }
-    download_cols(c, static_cast<const double*>(c.y.p), P.g.N_pad, N, K * v_count,
-                  [&](int64_t q0, int64_t nq, const double* p) {
-        for (int64_t q = q0; q < q0 + nq; ++q) {
-            if (!touched[(size_t)(q / v_count)]) continue;
-            T* dst = Xz + q * N;
-            const double* src = p + (q - q0) * N;
-            if (beta1[(size_t)(q / v_count)])
-                for (int64_t n = 0; n < N; ++n) dst[n] = (T)((double)dst[n] + src[n]);
-            else
-                for (int64_t n = 0; n < N; ++n) dst[n] = (T)src[n];
-        }
-    });
-    for (int64_t k = 0; bin_init && k < K; ++k)
-        if (touched[(size_t)k]) bin_init[k] = 1;
+    merge_sketch<T>(c.stage, c.st, static_cast<const double*>(c.y.p), P.g.N_pad, N, K, v_count,
+                    csr.nnz.data(), bin_init, Xz);
 }
 
 template <typename T>
@@ -1656,7 +1558,7 @@ void phase2_bed_impl(const char* bed_prefix, const char* fam_path, int blk_start
     const int64_t N = P.g.N, Np = P.g.N_pad;
     // Sketch to device (FP64, padded rows zero).
     double* dY = c.y.as<double>((size_t)(Np * Q));
-    upload_cols<T>(c, dY, Np, Xz, N, Q);
+    upload_cols<T>(c.stage, c.st, dY, Np, Xz, N, Q);
     if (Cm && Rm && p > 0) {
         // Work = ((I - C R) X)^T Xz = X^T (I - C R)^T Xz for the dense form
         // (gwldcore.cpp:2376-2390); the Mailman form projects the sketch,
@@ -3868,9 +3770,7 @@ LDS_API void lds_clear_device_cache(void) {
     if (c.pinned) cudaFreeHost(c.pinned);
     c.pinned = nullptr;
     c.pinned_n = 0;
-    if (c.stage) cudaFreeHost(c.stage);
-    c.stage = nullptr;
-    c.stage_n = 0;
+    c.stage.release();
 }
 
 #define P1_ARGS(T)                                                                              \

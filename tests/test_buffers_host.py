@@ -99,3 +99,51 @@ int main() {
     return bad("ok");
 }
 """) == "ok"
+
+
+# A block's contribution of several pieces (columns longer than a half; a last partial
+# piece) and of one: merged as the sketch's bins ask for, and not at all, nor marked
+# as written, where any of its copies fails.
+@needs_cuda_headers
+@pytest.mark.parametrize("N,K,v,fails", [(300007, 3, 13, [0, 1, 3, 38]), (60001, 3, 50, [0, 5]),
+                                         (60001, 3, 7, [0]), (500, 3, 7, [0])])
+def test_a_failed_download_leaves_the_sketch(tmp_path, N, K, v, fails):
+    assert run_cpp(tmp_path, r"""
+int main() {
+    const int64_t N = %d, K = %d, v = %d, ld = N + 5;
+    std::vector<double> d((size_t)(ld * K * v));
+    for (size_t i = 0; i < d.size(); ++i) d[i] = (double)(i %% 1013) - 500.0;
+    const std::vector<int64_t> nnz = {3, 5, 0};   // (the last bin has no members)
+    PinnedStage stage;
+    for (int f : {%s, -1}) {
+        std::vector<float> x((size_t)(N * K * v));
+        for (size_t i = 0; i < x.size(); ++i) x[i] = (float)(i %% 7);
+        const std::vector<float> before = x;
+        uint8_t init[3] = {0, 1, 0};
+        fail_copy = f;
+        bool threw = false;
+        try {
+            merge_sketch<float>(stage, nullptr, d.data(), ld, N, K, v, nnz.data(), init, x.data());
+        } catch (const Error&) { threw = true; }
+        if (threw != (f >= 0)) return bad("error not passed on");
+        if (threw && (x != before || init[0] != 0 || init[1] != 1)) return bad("changed");
+        if (threw) continue;
+        for (int64_t q = 0; q < K * v; ++q)
+            for (int64_t n = 0; n < N; ++n) {
+                const int64_t k = q / v;
+                const float old = before[(size_t)(q * N + n)], c = (float)d[(size_t)(q * ld + n)];
+                const float want = k == 0 ? c : k == 1 ? old + c : old;
+                if (x[(size_t)(q * N + n)] != want) return bad("wrong sum");
+            }
+        if (init[0] != 1 || init[1] != 1 || init[2] != 0) return bad("marks");
+    }
+    // and up again: pieces, the padding rows zero
+    std::vector<float> h((size_t)(N * K * v));
+    for (size_t i = 0; i < h.size(); ++i) h[i] = (float)(i %% 911);
+    upload_cols<float>(stage, nullptr, d.data(), ld, h.data(), N, K * v);
+    for (int64_t q = 0; q < K * v; ++q)
+        for (int64_t n = 0; n < ld; ++n)
+            if (d[(size_t)(q * ld + n)] != (n < N ? (double)h[(size_t)(q * N + n)] : 0.0)) return bad("upload");
+    return bad("ok");
+}
+""" % (N, K, v, ", ".join(map(str, fails)))) == "ok"
