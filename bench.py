@@ -528,10 +528,13 @@ def ours_arm(args) -> None:
     # phase-2 CTA order; every candidate's scores must agree bit for bit) ----
     from summit_b200 import autotune
 
-    cands = ([{"p1_sb_per_cta": s, "batch_gb": 8.0} for s in (8, 16, 32, 64, 128)] +
-             [{"p1_sb_per_cta": 64, "batch_gb": b} for b in (4.0, 16.0)] +
-             [{"p1_sb_per_cta": 128, "batch_gb": 8.0, "p2_bin_chunk": c} for c in (0, 12, 24)] +
-             [{"p1_sb_per_cta": 128, "batch_gb": 8.0, "p2_bin_chunk": 2, "p2_bins": 1}])
+    cands = ([dict(autotune.DEFAULT_CONFIG)] +
+             [{"p1_sb_per_cta": s, "batch_gb": 8.0} for s in (8, 16, 32, 64, 128)] +
+             [{"p1_sb_per_cta": s, "batch_gb": b} for s in (0, 64) for b in (4.0, 16.0)] +
+             [{"p1_sb_per_cta": s, "batch_gb": 8.0, "p2_bin_chunk": c}
+              for s in (0, 128) for c in (0, 12, 24)] +
+             [{"p1_sb_per_cta": s, "batch_gb": 8.0, "p2_bin_chunk": 2, "p2_bins": 1}
+              for s in (0, 128)])
     t_tune = time.perf_counter()
     tune = autotune.tune_windowed(sess, annot, ws, B_PROBES, BLOCK, PROBE_SEED, "rademacher",
                                   candidates=cands, reps=1)

@@ -40,12 +40,14 @@ DEFAULT_CONFIG = {"p1_sb_per_cta": 0, "batch_gb": 8.0, "p2_bin_chunk": 4, "p2_bi
 
 
 def default_candidates() -> list[dict]:
-    """Phase-1 split x window batching, then the phase-2 order and CTA shape."""
-    return ([{"p1_sb_per_cta": s, "batch_gb": b, "p2_bin_chunk": 4, "p2_bins": 0}
-             for s in (8, 16, 32, 64, 128) for b in (4.0, 8.0, 16.0)] +
-            [{"p1_sb_per_cta": 64, "batch_gb": 8.0, "p2_bin_chunk": c, "p2_bins": 0}
-             for c in (0, 12, 24)] +
-            [{"p1_sb_per_cta": 64, "batch_gb": 8.0, "p2_bin_chunk": 2, "p2_bins": 1}])
+    """The untuned configuration, phase-1 split (0: chosen per launch) x window
+    batching, then the phase-2 order and CTA shape with the chosen and a fixed
+    split."""
+    grid = [{"p1_sb_per_cta": s, "batch_gb": b, "p2_bin_chunk": 4, "p2_bins": 0}
+            for s in (0, 8, 16, 32, 64, 128) for b in (4.0, 8.0, 16.0)]
+    order = [{"p1_sb_per_cta": s, "batch_gb": 8.0, "p2_bin_chunk": c, "p2_bins": n}
+             for s in (0, 64) for c, n in ((0, 0), (12, 0), (24, 0), (2, 1))]
+    return [dict(DEFAULT_CONFIG)] + [c for c in grid if c != DEFAULT_CONFIG] + order
 
 
 def _apply(plan, cand: dict) -> None:

@@ -80,3 +80,27 @@ def test_default_candidates_cover_the_knobs():
     assert len({c["p1_sb_per_cta"] for c in cands}) >= 3
     assert all(set(c) == set(autotune.DEFAULT_CONFIG) for c in cands)
     assert {c["p2_bins"] for c in cands} == {0, 1}
+
+
+# An untuned plan takes DEFAULT_CONFIG, whose phase-1 split is chosen per launch: a
+# tuned plan must not be worse, so the tuner times it, and first; the phase-2 knobs
+# are tried with that split too.
+def test_the_untuned_configuration_is_a_candidate():
+    cands = autotune.default_candidates()
+    assert cands[0] == autotune.DEFAULT_CONFIG and cands.count(autotune.DEFAULT_CONFIG) == 1
+    for key in ("batch_gb", "p2_bin_chunk", "p2_bins"):
+        assert {c[key] for c in cands if c["p1_sb_per_cta"] == 0} == {c[key] for c in cands}
+    assert len({tuple(sorted(c.items())) for c in cands}) == len(cands)
+
+
+def test_the_bench_times_the_untuned_configuration():
+    import ast
+    from pathlib import Path
+
+    tree = ast.parse((Path(__file__).resolve().parents[1] / "bench.py").read_text())
+    lists = [n.value for n in ast.walk(tree) if isinstance(n, ast.Assign)
+             and [getattr(t, "id", "") for t in n.targets] == ["cands"]]
+    assert lists
+    for node in lists:
+        cands = eval(compile(ast.Expression(node), "bench.py", "eval"), {"autotune": autotune})
+        assert cands[0] == autotune.DEFAULT_CONFIG
