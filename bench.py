@@ -150,11 +150,25 @@ def reference_sample(m_sample: int, tmpdir: str, packed=None) -> tuple[str, np.n
     return prefix, annotations(M_SNPS)[:m_sample]
 
 
-def reference_built() -> bool:
-    """Whether the reference's own gwldcore.cpp has been compiled here (oracle/_ref)."""
-    from oracle.oracle import REF_SO
+NO_REFERENCE = "the reference's CPU library is not built (make -C oracle ref needs its sources)"
 
-    return REF_SO.exists()
+
+def reference_built(library: str = "REF_SO") -> bool:
+    """Whether the reference's own code (gwldcore.cpp; REF_WIN_SO winldcore.cpp,
+    REF_GXE_SO gxeldcore.cpp) has been compiled here (oracle/_ref)."""
+    from oracle import oracle
+
+    return getattr(oracle, library).exists()
+
+
+def cpu_baseline_missing(line: dict, library: str) -> bool:
+    """Whether there is no CPU baseline to take; says why in `line`."""
+    if os.environ.get("LDS_SKIP_CPU_BASELINE"):
+        return True
+    if not reference_built(library):
+        line["cpu_baseline"] = {"unavailable": NO_REFERENCE}
+        return True
+    return False
 
 
 def run_reference_windows(packed: np.ndarray, annot: np.ndarray, ws: np.ndarray, threads: int,
@@ -257,6 +271,9 @@ def reference_sample_windows(target_s: float, threads: int, tmpdir: str, packed=
 def reference_arm(args) -> None:
     rank = env_int("RANK", 0)
     if rank != 0:
+        return
+    if not reference_built():
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
         return
     threads = cpu_threads()
     os.environ.setdefault("OMP_NUM_THREADS", str(threads))
@@ -701,10 +718,7 @@ def ours_arm(args) -> None:
             line["product_checks"] = product_checks
         if lvp is not None:
             line["learned_vs_plain"] = lvp
-        if world == 1 and not reference_built():
-            line["cpu_baseline"] = {"unavailable": "the reference's CPU library is not built "
-                                                   "(make -C oracle ref needs its sources)"}
-        elif world == 1 and not os.environ.get("LDS_SKIP_CPU_BASELINE"):
+        if world == 1 and not cpu_baseline_missing(line, "REF_SO"):
             threads = cpu_threads()
             with tempfile.TemporaryDirectory() as td:
                 pk, ann_s, ws_s = reference_sample_windows(
@@ -808,7 +822,7 @@ def exact_arm(args) -> None:
                                          else "fallback"),
                          "traffic": None, "algorithmic_ops_per_launch": ops},
             "gpu_launches": launches, "clocks": clk.summary()}
-    if not os.environ.get("LDS_SKIP_CPU_BASELINE"):
+    if not cpu_baseline_missing(line, "REF_WIN_SO"):
         from oracle.oracle import ReferenceWindowed
         from summit_b200 import bedfile
 
@@ -969,7 +983,7 @@ def gxe_arm(args) -> None:
             "unchecked_target_ms": round(res["timings"]["target"], 1),
             "rows": rc["rows"], "mismatches": rc["mismatches"], "scores_identical": bool(same)}
         gxc.close()
-    if rank == 0 and world == 1 and not os.environ.get("LDS_SKIP_CPU_BASELINE"):
+    if rank == 0 and world == 1 and not cpu_baseline_missing(line, "REF_GXE_SO"):
         threads = cpu_threads()
         snps = env_int("LDS_GXE_CPU_SNPS", 400)
         sec, sample = gxe_reference_sample(n, snps, threads)
@@ -1294,7 +1308,7 @@ def biobank_arm(args) -> None:
                      "memory; the image is generated on the device"),
         "gpu_launches": launches, "clocks": clk.summary(),
     }
-    if not os.environ.get("LDS_SKIP_CPU_BASELINE"):
+    if not cpu_baseline_missing(line, "REF_SO"):
         # The reference's per-block native calls (gwldcore.cpp, compiled
         # unchanged) on the leading SNPs of the same data (the generator's
         # first L SNPs do not depend on M).
@@ -1348,7 +1362,9 @@ def main() -> None:
             return
         generalized_arm(args)
     elif args.workload == "gxe":
-        if args.impl == "reference":
+        if args.impl == "reference" and not reference_built("REF_GXE_SO"):
+            print(json.dumps({"impl": "reference", "workload": "gxe", "unavailable": NO_REFERENCE}))
+        elif args.impl == "reference":
             sec, sample = gxe_reference_sample(GXE_N, env_int("LDS_GXE_CPU_SNPS", 400),
                                                cpu_threads())
             v = gxe_ops(GXE_N, env_int("LDS_GXE_CPU_SNPS", 400), GXE_E, 1, GXE_B) / sec / 1e12
