@@ -199,24 +199,34 @@ __global__ void gen_rows_kernel(const long long* __restrict__ raw_g,
 }
 
 // directed[c1][c2] += sum_jl a[j0 + jl][k1] rows[jl][p1][c2], c1 = k1 P + p1,
-// in two steps: sums over chunks of kDirRows variants (one CTA each), then one
-// warp per entry over the chunks, both in a fixed order.  One thread per entry
-// over all variants left the chip idle: C = 6, 6,000 variants 786 -> 25 us.
-constexpr int kDirRows = 64;
+// in two steps: sums over chunks of variants, then one warp per entry over the
+// chunks, both in a fixed order.  A CTA takes 256 entries of a chunk; the chunks are
+// of at least kDirRows variants, and as many as give kDirCtas CTAs, which also bounds
+// their sums (one CTA for all entries of a chunk left C = 291 with 94 CTAs).
+// 6,000 variants, C = 6: 786 -> 25 us (one thread per entry over all variants);
+// C = 291: 883 us (1,298; with one CTA per chunk 3,597).
+constexpr int kDirRows = 64, kDirThreads = 256, kDirCtas = 8 * 148;
 
-__global__ void gen_directed_kernel(const double* __restrict__ rows, int64_t L,
-                                    const double* __restrict__ annot, int64_t j0, int K, int P,
-                                    double* __restrict__ part) {
-    const int C = K * P;
-    const int64_t r0 = (int64_t)blockIdx.x * kDirRows, r1 = min(L, r0 + kDirRows);
-    for (int idx = threadIdx.x; idx < C * C; idx += blockDim.x) {
-        const int c1 = idx / C, c2 = idx - c1 * C, k1 = c1 / P, p1 = c1 - k1 * P;
-        double s = 0.0;
+// Chunks of L variants for n entries.
+static int64_t gen_directed_chunks(int64_t L, int64_t n) {
+    const int64_t groups = (n + kDirThreads - 1) / kDirThreads;
+    return std::max<int64_t>(1, std::min((L + kDirRows - 1) / kDirRows,
+                                         (kDirCtas + groups - 1) / groups));
+}
+
+__global__ void __launch_bounds__(kDirThreads)
+    gen_directed_kernel(const double* __restrict__ rows, int64_t L, int64_t rows_per_chunk,
+                        const double* __restrict__ annot, int64_t j0, int K, int P,
+                        double* __restrict__ part) {
+    const int C = K * P, idx = (int)(blockIdx.x * kDirThreads + threadIdx.x);
+    if (idx >= C * C) return;
+    const int64_t r0 = (int64_t)blockIdx.y * rows_per_chunk, r1 = min(L, r0 + rows_per_chunk);
+    const int c1 = idx / C, c2 = idx - c1 * C, k1 = c1 / P, p1 = c1 - k1 * P;
+    double s = 0.0;
 #pragma unroll 8
-        for (int64_t jl = r0; jl < r1; ++jl)
-            s += annot[(j0 + jl) * K + k1] * rows[(jl * P + p1) * C + c2];
-        part[(int64_t)blockIdx.x * C * C + idx] = s;
-    }
+    for (int64_t jl = r0; jl < r1; ++jl)
+        s += annot[(j0 + jl) * K + k1] * rows[(jl * P + p1) * C + c2];
+    part[(int64_t)blockIdx.y * C * C + idx] = s;
 }
 
 __global__ void gen_directed_reduce_kernel(const double* __restrict__ part, int64_t nchunks, int n,
@@ -367,18 +377,20 @@ void launch_gen_rows(const long long* raw_g, const long long* raw_o, int64_t raw
 }
 
 int64_t gen_directed_part_elems(int64_t L, int K, int P) {
-    return (L + kDirRows - 1) / kDirRows * K * P * K * P;
+    const int64_t n = (int64_t)K * P * K * P;
+    return gen_directed_chunks(L, n) * n;
 }
 
 void launch_gen_directed(const double* rows, int64_t L, const double* annot, int64_t j0, int K,
                          int P, double* part, double* directed, cudaStream_t st) {
-    const int C = K * P;
+    const int C = K * P, n = C * C;
     if (L <= 0 || C <= 0) return;
-    const int64_t chunks = (L + kDirRows - 1) / kDirRows;
-    gen_directed_kernel<<<(unsigned)chunks, 256, 0, st>>>(rows, L, annot, j0, K, P, part);
+    const int64_t chunks = gen_directed_chunks(L, n), per = (L + chunks - 1) / chunks;
+    const int64_t used = (L + per - 1) / per;
+    gen_directed_kernel<<<dim3((unsigned)((n + kDirThreads - 1) / kDirThreads), (unsigned)used),
+                          kDirThreads, 0, st>>>(rows, L, per, annot, j0, K, P, part);
     count_launch();
-    gen_directed_reduce_kernel<<<(unsigned)((C * C + 7) / 8), 256, 0, st>>>(part, chunks, C * C,
-                                                                           directed);
+    gen_directed_reduce_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(part, used, n, directed);
     count_launch();
 }
 

@@ -78,3 +78,35 @@ def test_gxe_shared_tiles(m, T, B):
     for c in range(T * 2 * B):   # (column by column: a wrong one among many shows)
         assert rel_err(out[0][:, c], out[1][:, c]) < 1e-6
     sess.close()
+
+
+# The directed numerator's split over variants and entries (chunks of 64 variants; ten
+# chunks of 90; two blocks of variants, whose sums add up), against the sum over the
+# scores that the same call returns: FP64 sums of at most 900 terms.
+@pytest.mark.parametrize("K,Q,m,width", [(2, 2, 130, 130), (60, 2, 900, 900), (97, 1, 700, 500)])
+def test_directed_numerator_forms(K, Q, m, width):
+    from conftest import rel_err
+    from summit_b200 import bedfile, generalized_gxe as gg
+    from summit_b200.session import GwSession
+
+    n, B = 64, 2
+    rng = np.random.default_rng(K)
+    sess = GwSession(bedfile.pack_bed_rows(rng.binomial(2, 0.4, (m, n)).astype(np.int8)), n)
+    pairs = gg.pair_order(Q)
+    term_off, term_f1, term_f2 = [0], [], []
+    for tp in pairs:
+        for sp in pairs:
+            for tl, tr in gg._orientations(tp):
+                for sl, sr in gg._orientations(sp):
+                    term_f1.append(tr * Q + sl)
+                    term_f2.append(tl * Q + sr)
+            term_off.append(len(term_f1))
+    to, f1, f2 = (np.asarray(x, np.int32) for x in (term_off, term_f1, term_f2))
+    annot = rng.uniform(0.0, 1.0, size=(m, K))
+    rhs = np.asfortranarray(rng.normal(size=(n, K * B * Q * Q)))
+    P = len(pairs)
+    directional, directed = gg._pass2_scores(sess, rhs, K, B, Q * Q, P, to, f1, f2, float(n - 1),
+                                             annot, width)
+    want = np.einsum("vk,vpc->kpc", annot, directional.reshape(m, P, K * P)).reshape(K * P, K * P)
+    assert rel_err(directed.reshape(K * P, K * P), want) < 1e-12
+    sess.close()
