@@ -139,8 +139,8 @@ void launch_gram_reduce(const double* units, const int32_t* beg, const int32_t* 
 void launch_gxe_source_finalize(const double* Y, int64_t N, int64_t N_pad, int64_t C, int cols_half,
                                 const double* env, int64_t env_ld, int env_start, double* target,
                                 int64_t t_ld, cudaStream_t st);
-// out[c nb + a] = basis_a . panel_c (basis null: column sums, nb = 1); with
-// `squares` out[c] = panel_c . panel_c.  nb <= col_dots_max_basis().
+// out[c nb + a] = basis_a . panel_c, nb <= col_dots_max_basis(); with `squares`
+// (basis unused, nb = 1) out[c] = panel_c . panel_c.
 // (columns [g group_cols, (g + 1) group_cols) use the basis at basis + g group_stride)
 void launch_col_dots(const double* panel, int64_t p_ld, int64_t N, int64_t C, const double* basis,
                      int64_t b_ld, int nb, int squares, double* out, cudaStream_t st,

@@ -39,7 +39,6 @@ constexpr int kR = 32;         // rows per tile
 constexpr int kThreads = 256;  // threads of a tile's group
 constexpr int kMaxGroups = 4;  // groups per CTA (forward)
 
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float gelu(float z) {
     return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
 }

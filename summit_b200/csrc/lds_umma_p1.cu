@@ -11,7 +11,7 @@
 // accumulator, so TMEM holds G.W1 - O.W2 = sum_j (g - mu_j o) s_j sc z directly.
 //
 // Roles (832 threads): warp 0 TMA producer for the digit tiles; warp 1 TMEM
-// allocation and the single MMA-issuing thread; warps 2-9, four decoder sets of
+// allocation and MMA issue (one elected thread); warps 2-9, four decoder sets of
 // two (set d takes the K-steps it with it % 4 == d), gather the member SNPs' packed
 // bytes from global memory (one row each, kept several steps ahead by
 // cp.async) and decode them into the operand tiles; warps 10-25, eight per TMEM
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(kWarp ? 32 * kWWarps : kWMaxThreads)
     const int64_t r0 = w.bin_off[k], nnzp = w.bin_off[k + 1] - r0;
     const int64_t stride = (int64_t)nranks * gsize * 4;
     const int64_t rbeg = ((int64_t)rank * gsize + gtid) * 4;
-    // Members r .. r + 3 (lists are padded to a multiple of 128): w1 and mu w1.
+    // Members r .. r + 3 (lists are padded to a multiple of kP1Step): w1 and mu w1.
     auto load4 = [&](int64_t r, double (&a)[4], double (&m)[4]) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -751,7 +751,7 @@ void launch_p1_umma(const P1UArgs& a, int64_t N_pad, cudaStream_t st) {
     b.sb_per_cta = std::max(std::min(a.sb_per_cta, p1::kMaxSb) / b.share, 1) * b.share;
     dim3 grid((unsigned)(N_pad / p1::kBM), (unsigned)((a.K + b.sb_per_cta - 1) / b.sb_per_cta));
     // Few sample tiles leave SMs idle while each CTA walks its whole list: as
-    // many CTAs as fill the chip once then share a list's K-steps (8 at least
+    // many CTAs as fill the chip once then share a list's K-steps (16 at least
     // each).  Their contributions are integers times the column's power-of-two
     // scale, all below 2^53 in total, so the FP64 additions into the zeroed
     // sketch are exact in any order.  N = 5,000 (40 tiles), K = 1, 20,000

@@ -280,7 +280,7 @@ class WinPlan:
 
     # ---- control-variate outputs (see lds_win_plan_set_cv) ----
     def set_tiling(self, p1_sb_per_cta: int = 0) -> None:
-        """Phase-1 super-bins per CTA (0: default); call before the first
+        """Phase-1 super-bins per CTA (0: chosen from the member lists); call before the first
         execute."""
         check(_lib.load().lds_win_plan_set_tiling(self.handle, int(p1_sb_per_cta)))
 
