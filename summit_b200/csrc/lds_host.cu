@@ -1815,7 +1815,7 @@ std::unique_ptr<GwPlan> plan_create(Context& c, std::shared_ptr<Prepared> P, con
             for (int64_t kk = 0; kk < K; ++kk)
                 t->lmax = std::max(t->lmax, cs.bin_off[(size_t)kk + 1] - cs.bin_off[(size_t)kk]);
             t->p1_sb = umma::choose_sb_per_cta(cs.bin_off.data(), (int)K, umma::ncolp_for(V),
-                                               P->g.N_pad / 128, (int)K);
+                                               P->g.N_pad / 128, (int)K, 1);
             t->wq.as<int8_t>(std::max<size_t>(
                 umma::w_digit_bytes(cs.bin_off[(size_t)K], umma::ncolp_for(V)), 16));
             t->wcs.as<double>((size_t)(K * V));
@@ -2397,7 +2397,8 @@ std::unique_ptr<WinPlan> win_plan_create(Context& c, std::shared_ptr<Prepared> P
         cs.bin_off[(size_t)b.ksup] = off;
         for (int V : pl->vt)
             b.p1_sb.push_back(umma::choose_sb_per_cta(cs.bin_off.data(), (int)b.ksup,
-                                                      umma::ncolp_for(V), Np / 128, (int)K));
+                                                      umma::ncolp_for(V), Np / 128, (int)K,
+                                                      umma::kPlainWindowed));
         const size_t nm = std::max<size_t>(ri.size(), 1);
         h2d(b.rowind.as<int32_t>(nm), ri.data(), ri.size(), c.st);
         h2d(b.sc.as<double>(nm), scv.data(), scv.size(), c.st);

@@ -28,7 +28,7 @@ int main() {
     const int K = %d, W = %d, members = %d;
     std::vector<int64_t> off{0};
     for (int q = 0; q < K * W; ++q) off.push_back(off.back() + members);
-    std::printf("%%d", lds::umma::choose_sb_per_cta(off.data(), K * W, %d, %d, K));
+    std::printf("%%d", lds::umma::choose_sb_per_cta(off.data(), K * W, %d, %d, K, %d));
 }
 """
 
@@ -38,25 +38,32 @@ int main() {
 @pytest.mark.parametrize("K", [67, 97, 134])
 @pytest.mark.parametrize("W,tiles", [(20, 40), (700, 391)])
 def test_bins_with_few_divisors_share_a_cta(tmp_path, K, W, tiles):
-    assert int(run_cpp(tmp_path, SHAPE % (K, W, 128, 208, tiles))) >= 8
+    assert int(run_cpp(tmp_path, SHAPE % (K, W, 128, 208, tiles, 8))) >= 8
 
 
 # The super-bins' CTAs lie along grid.y, which holds 65,535: 97 bins x 700 windows
 # at one per CTA would not fit, nor 24 x 3,000 (or x 200,000) at few per CTA.
 @pytest.mark.parametrize("K,W", [(97, 700), (24, 3000), (1, 70000), (24, 200000)])
 def test_the_grid_holds_the_ctas(tmp_path, K, W):
-    s = int(run_cpp(tmp_path, SHAPE % (K, W, 64, 48, 2)))
+    s = int(run_cpp(tmp_path, SHAPE % (K, W, 64, 48, 2, 8)))
     assert 1 <= s <= 256 and -(-K * W // s) <= 65535
 
 
-# 8 windows x 23 bins over 40 sample tiles: whole windows are estimated 2.6 %
-# earlier than 8 per CTA, within the estimate's own error.
-def test_a_near_tie_keeps_the_plain_number(tmp_path):
-    assert int(run_cpp(tmp_path, SHAPE % (23, 8, 128, 80, 40))) == 8
+# 8 windows x 23 bins over 40 sample tiles, and one window of 13 over 79: whole windows
+# are estimated up to 2.6 % earlier than 8 per CTA, within the estimate's own error.
+@pytest.mark.parametrize("K,W,members,ncolp,tiles", [(23, 8, 128, 80, 40), (13, 1, 192, 48, 79)])
+def test_a_near_tie_keeps_the_plain_number(tmp_path, K, W, members, ncolp, tiles):
+    assert int(run_cpp(tmp_path, SHAPE % (K, W, members, ncolp, tiles, 8))) == 8
+
+
+# A genome-wide plan (plain number 1) gains no candidate by that.
+def test_genome_wide_numbers_are_divisors(tmp_path):
+    assert int(run_cpp(tmp_path, SHAPE % (11, 1, 2048, 80, 79, 1))) in (1, 11)
+    assert int(run_cpp(tmp_path, SHAPE % (24, 1, 4096, 208, 391, 1))) == 8
 
 
 def test_even_parts_of_a_window(tmp_path):
-    assert int(run_cpp(tmp_path, SHAPE % (24, 60, 128, 208, 391))) in (8, 12, 24, 48)
+    assert int(run_cpp(tmp_path, SHAPE % (24, 60, 128, 208, 391, 8))) in (8, 12, 24, 48)
 
 
 DIGITS = """
